@@ -37,15 +37,18 @@ typedef struct orkan_qaoa orkan_qaoa_t;
  *   mem_budget         device bytes the batch may use for state vectors (0: 60 % of the free
  *                      memory after the cost vectors); instances are evaluated in waves that fit
  *   flags              ORKAN_QAOA_* flags
+ * A cut's cost and the whole circuit are unchanged when every bit is flipped, so an instance of
+ * more qubits than a chunk holds keeps the 2^(n-1) amplitudes whose top bit is clear.
  * Instances with the same qubit count, edge list and weights share one resident cost vector
- * (2^n bytes for byte costs, plus a transposed copy of the same size that the high passes
- * read; 2^n doubles for FP64 costs).  All arrays are host arrays, copied. */
+ * (2^(n-1) costs in the order of the low passes and as many in that of the high ones; bytes, or
+ * doubles for FP64 costs).  All arrays are host arrays, copied. */
 int orkan_qaoa_create(orkan_qaoa_t **out, unsigned count, const unsigned *n_qubits, const unsigned *edge_offsets,
                       const unsigned *edges, const double *weights, unsigned p, unsigned long long mem_budget,
                       unsigned flags);
 
 /* Evaluate every instance: gammas and betas are host arrays [count][p] in instance order;
- * means[i] receives the expectation value of the cost.  Synchronises the stream. */
+ * means[i] receives the expectation value of the cost.  Synchronises the stream.  Returns
+ * cudaErrorLaunchTimeout when a kernel's bounded wait for staged data ran out. */
 int orkan_qaoa_run(orkan_qaoa_t *b, const double *gammas, const double *betas, double *means, void *stream);
 
 /* Autotune chunk size, block size and buffer depth per qubit count on this batch (timing
@@ -56,8 +59,8 @@ int orkan_qaoa_run(orkan_qaoa_t *b, const double *gammas, const double *betas, d
 int orkan_qaoa_tune(orkan_qaoa_t *b, const double *gammas, const double *betas, const char *cache_path);
 
 /* Current launch configuration of instances of n qubits: log2 of the chunk (amplitudes per
- * work item), threads per block, and the number of shared buffers per block (2: the next
- * item is copied in while the current one computes). */
+ * work item), threads that compute one item, and the buffer depth (2: the next items are
+ * copied in while the current ones are computed). */
 int orkan_qaoa_config(const orkan_qaoa_t *b, unsigned n, unsigned *log_chunk, unsigned *threads, unsigned *ring);
 
 /* Copy the device cost vector of instance i (2^n doubles) to host memory (for checks). */

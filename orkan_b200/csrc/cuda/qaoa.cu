@@ -20,111 +20,297 @@ using namespace orkan;
 
 namespace {
 
-// cost[x] = sum_e w_e [bit u_e of x != bit v_e of x], edges in the given order.
+// One graph's place in the resident arrays: its edges and weights, and its costs.
+struct QaoaEdges {
+    const unsigned char* uv;
+    const double* w;
+    unsigned ne;
+};
+
+// Costs of one kind of pass in its order (qaoa_cost_slot):
+// cost[i] = sum_e w_e [bit u_e of x != bit v_e of x], x = qaoa_cost_state(i), edges in the
+// given order.
 template <class CostT>
-__global__ void k_qaoa_cost(CostT* cost, unsigned n, const unsigned char* edges, const double* w, unsigned ne) {
-    const idx_t dim = idx_t(1) << n;
-    for (idx_t x = (idx_t)blockIdx.x * blockDim.x + threadIdx.x; x < dim; x += (idx_t)gridDim.x * blockDim.x) {
+__global__ void k_qaoa_cost(CostT* cost, QaoaGeo g, idx_t count, QaoaEdges E) {
+    for (idx_t i = (idx_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (idx_t)gridDim.x * blockDim.x) {
+        const unsigned x = (unsigned)qaoa_cost_state(g, sizeof(CostT) == 1, i);
         double c = 0.0;
-        for (unsigned e = 0; e < ne; ++e)
-            if (((x >> edges[2 * e]) ^ (x >> edges[2 * e + 1])) & 1u) c += w[e];
-        cost[x] = (CostT)c;
+        for (unsigned e = 0; e < E.ne; ++e)
+            if (((x >> E.uv[2 * e]) ^ (x >> E.uv[2 * e + 1])) & 1u) c += E.w[e];
+        cost[i] = (CostT)c;
     }
 }
 
-// Transposed byte costs for the high passes of chunks of 2^C: dst[col 2^R + row] =
-// src[row 2^C + col] with R = n - C (qaoa_cost_t_index), through 32 x 32 tiles in shared
-// memory so that reads and writes are both runs of consecutive bytes.
-__global__ void k_qaoa_cost_transpose(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, unsigned n,
-                                      unsigned C) {
-    __shared__ uint8_t tile[32][33];
-    const idx_t rows = idx_t(1) << (n - C), cols = idx_t(1) << C;
-    const idx_t tiles_c = (cols + 31) / 32, tiles = ((rows + 31) / 32) * tiles_c;
-    for (idx_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const idx_t r0 = (t / tiles_c) * 32, c0 = (t % tiles_c) * 32;
-        for (unsigned i = threadIdx.y; i < 32; i += blockDim.y) {
-            const idx_t r = r0 + i, c = c0 + threadIdx.x;
-            if (r < rows && c < cols) tile[i][threadIdx.x] = src[r * cols + c];
-        }
-        __syncthreads();
-        for (unsigned i = threadIdx.y; i < 32; i += blockDim.y) {
-            const idx_t c = c0 + i, r = r0 + threadIdx.x;
-            if (r < rows && c < cols) dst[c * rows + r] = tile[threadIdx.x][i];
-        }
-        __syncthreads();
+// The whole cost vector from the resident costs of the low (or full) passes.
+template <class CostT>
+__global__ void k_qaoa_cost_vector(const CostT* cost, QaoaGeo g, idx_t count, double* out) {
+    const idx_t all = (idx_t(1) << g.n) - 1;
+    for (idx_t i = (idx_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (idx_t)gridDim.x * blockDim.x) {
+        const idx_t x = qaoa_cost_state(g, sizeof(CostT) == 1, i);
+        out[x] = (double)cost[i];
+        if (g.kind != kQaoaFull) out[all ^ x] = (double)cost[i];
     }
 }
 
-// table[(pos p + k) tstride + c] = (cos, sin)(c * gamma[pos p + k]) for c <= cmax of pos
-__global__ void k_qaoa_tables(const unsigned* cmax, const double* gamma, unsigned count, unsigned p,
+// table[(pos p + k) tstride + c] = fs (cos, sin)(c * gamma[pos p + k]) for c <= cmax of pos
+__global__ void k_qaoa_tables(const unsigned* cmax, const double* gamma, const QaoaRx* rx, unsigned count, unsigned p,
                               unsigned tstride, double2* table) {
     const unsigned pos = blockIdx.x;
     if (pos >= count || cmax[pos] >= kQaoaMaxTable) return;
     const unsigned m = cmax[pos] + 1;
     for (unsigned t = threadIdx.x; t < p * m; t += blockDim.x) {
         const unsigned k = t / m, c = t % m;
+        const idx_t row = (idx_t)pos * p + k;
+        const double fs = rx[row].fs;
         double sn, cs;
-        sincos((double)c * gamma[(idx_t)pos * p + k], &sn, &cs);
-        table[((idx_t)pos * p + k) * tstride + c] = c2(cs, sn);
+        sincos((double)c * gamma[row], &sn, &cs);
+        table[row * tstride + c] = c2(cs * fs, sn * fs);
     }
 }
 
-// Persistent pass kernel: each block walks the work items w = blockIdx.x, + gridDim.x, ...
-// With RING = 2 the next item's amplitudes and costs are copied asynchronously into the
-// second shared buffer while the current item is computed; with RING = 1 (2^13-amplitude
-// chunks, which leave no room for a second buffer) the copy follows the item.
-template <unsigned NT, class CostT, unsigned RING>
-__global__ void __launch_bounds__(NT, 65536 / (NT * 128)) k_qaoa_pass(QaoaPass P, QaoaTables T) {
-    extern __shared__ __align__(16) unsigned char smem_q[];
-    const unsigned lc = P.kind == kQaoaFull ? P.plan.q1 : P.C;
-    const idx_t cmask = (idx_t(1) << P.li) - 1;
-    auto fill = [&](idx_t w, unsigned slot) {
-        const QaoaInst I = P.inst[w >> P.li];
-        const QaoaPlan& pl = P.plan;
-        const QaoaSmem<CostT> S = qaoa_smem_at<CostT>(smem_q, lc, NT, RING, slot);
-        qaoa_fill<CostT>(P, T, I, pl, QaoaDevPsi{I.psi}, QaoaDevCost<CostT>{static_cast<const CostT*>(I.cost)},
-                         w & cmask, S, threadIdx.x, NT);
-    };
-    unsigned slot = 0;
-    idx_t w = blockIdx.x;
-    if (w < P.items) fill(w, 0);
-    qaoa_cp_commit();
-    for (; w < P.items; w += gridDim.x) {
-        const idx_t wn = w + gridDim.x;
-        if (RING == 2) {
-            if (wn < P.items) fill(wn, slot ^ 1u);
-            qaoa_cp_commit();
-            qaoa_cp_wait<1>();
+// ---- device accessors ------------------------------------------------------------------
+__device__ __forceinline__ unsigned sm_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+struct QaoaDevPsi {
+    double2* p;
+    __device__ __forceinline__ void st(idx_t i, double2 v) const { p[i] = v; }
+    __device__ __forceinline__ void cp16(double2* dst, idx_t i) const {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sm_u32(dst)), "l"(p + i) : "memory");
+    }
+    __device__ __forceinline__ void bulk_load(double2* dst, idx_t i, unsigned n, void* bar) const {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                     ::"r"(sm_u32(dst)), "l"(p + i), "r"(n * 16u), "r"(sm_u32(bar)) : "memory");
+    }
+};
+template <class CostT>
+struct QaoaDevCost;
+template <>
+struct QaoaDevCost<double> {
+    const double* p;
+    __device__ __forceinline__ double ld(unsigned i) const { return __ldg(p + i); }
+};
+template <>
+struct QaoaDevCost<uint8_t> {
+    const uint8_t* p;
+    __device__ __forceinline__ uint8_t ld(unsigned i) const { return __ldg(p + i); }
+    // the 2^K costs at i, a multiple of 2^K
+    template <int K>
+    __device__ __forceinline__ void words(uint32_t* w, unsigned i) const {
+        if constexpr (K == 4) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p + i));
+            w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        } else if constexpr (K == 3) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + i));
+            w[0] = v.x; w[1] = v.y;
+        } else if constexpr (K == 2) {
+            w[0] = __ldg(reinterpret_cast<const unsigned*>(p + i));
         } else {
-            qaoa_cp_wait<0>();
-        }
-        __syncthreads();
-        const QaoaInst I = P.inst[w >> P.li];
-        const QaoaPlan& pl = P.plan;
-        const QaoaSmem<CostT> S = qaoa_smem_at<CostT>(smem_q, lc, NT, RING, slot);
-        const unsigned nst = qaoa_stages(pl);
-        for (unsigned st = 0; st < nst; ++st) {
-            qaoa_stage<CostT>(P, T, I, pl, QaoaDevPsi{I.psi}, w & cmask, st, S, threadIdx.x, NT);
-            __syncthreads();
-        }
-        if (RING == 2) {
-            slot ^= 1u;
-        } else {
-            if (wn < P.items) fill(wn, 0);
-            qaoa_cp_commit();
+            w[0] = __ldg(reinterpret_cast<const unsigned short*>(p + i));
         }
     }
-    qaoa_cp_wait<0>();
+};
+
+__device__ __forceinline__ void mb_init(void* bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(sm_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mb_arrive(void* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(sm_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void mb_expect(void* bar, unsigned bytes) {
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;\n" ::"r"(sm_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mb_try(void* bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                 " selp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(ok) : "r"(sm_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Bounded wait: false when the limit is reached.
+__device__ __forceinline__ bool mb_wait(void* bar, unsigned parity, unsigned long long limit) {
+    for (unsigned long long i = 0; i < limit; ++i)
+        if (mb_try(bar, parity)) return true;
+    return false;
 }
 
-// out[pos] = sum of the instance's chunk partials, in chunk order
-__global__ void k_qaoa_fold(const QaoaInst* inst, unsigned ninst, const double* partial, idx_t items, double* out) {
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ninst) return;
+// Shape of a pass block by chunk size: `groups` groups of 2^C / 16 threads work on one item
+// each, and the other buffers hold staged items.  Four more warps stage the items.
+//
+// Registers: a block of 640 threads is launched with 96 each (61440); the staging warps give
+// back all but 32 (4096 in all) and the computing ones then take 112 (57344), which holds the
+// 16 amplitudes of a set (64) with little spilled.
+constexpr unsigned kStageThreads = 128;
+constexpr unsigned kComputeThreads = 512;
+constexpr unsigned kLaunchRegs = 96, kStageRegs = 32, kComputeRegs = 112;
+static_assert(kStageThreads * kStageRegs + kComputeThreads * kComputeRegs <=
+              (kStageThreads + kComputeThreads) * kLaunchRegs, "register split within the launch's registers");
+template <unsigned C>
+struct PassShape {
+    static constexpr unsigned kThreads = (1u << C) / 16;
+    static constexpr unsigned kGroups = kComputeThreads / kThreads;
+    static constexpr unsigned kBuffers = C >= 13 ? 1 : kGroups + kGroups / 2;
+    static constexpr unsigned kBlock = kComputeThreads + kStageThreads;
+};
+
+// One pass over the items of a launch.  Block b takes items b, b + grid, ... in turn; group g
+// computes every kGroups-th of them, and the staging warp keeps the free buffers filled: low
+// items by one bulk copy of 2^C amplitudes, high items by 16-byte copies of runs.  A group
+// hands its buffer back as soon as its last stage has its amplitudes in registers.
+//
+// Bound: HBM (32 bytes per stored amplitude in a middle pass) and shared memory (2 m - 1
+// stages of 32 bytes) are close at C = 12; the registers of the 16 computing warps leave one
+// block per SM, so the copies run ahead of the arithmetic instead of in another block.
+// Measured (16 instances, p = 4, ms per run) against two 256-thread blocks per SM that filled,
+// computed and stored one item after the other on the whole state: 24 qubits 5.61 against
+// 17.17, 22 qubits 1.41 against 4.13, 20 qubits 0.41 against 0.95, 16 qubits 0.086 against
+// 0.098; 8 weighted instances of 24 qubits at p = 6 6.60 against 19.8.  Half of the state's
+// amplitudes account for a factor of two, the staging and the shorter stages for the rest.
+template <class CostT, unsigned C>
+__global__ void __launch_bounds__(PassShape<C>::kBlock, 1)
+    k_qaoa_pass(const __grid_constant__ QaoaPass P, const QaoaTables T) {
+    using Sh = PassShape<C>;
+    constexpr unsigned NB = Sh::kBuffers, GT = Sh::kThreads, NG = Sh::kGroups;
+    constexpr bool kBytes = sizeof(CostT) == 1;
+    extern __shared__ __align__(128) unsigned char smem_q[];
+    const QaoaSmem L = qaoa_smem(C, NB, kBytes ? T.tstride : 0u, 512);
+    unsigned long long* full = reinterpret_cast<unsigned long long*>(smem_q + L.bar);
+    unsigned long long* empty = full + NB;
+    unsigned char* flags = reinterpret_cast<unsigned char*>(empty + NB);
+    if (threadIdx.x == 0) {
+        for (unsigned b = 0; b < NB; ++b) {
+            mb_init(full + b, kStageThreads + 1);      // the staging threads' copies, and the first one
+            mb_init(empty + b, GT / 32);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    const unsigned warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const unsigned items = (unsigned)P.items;          // checked to fit by the host
+    if (warp >= kComputeThreads / 32) {                // staging
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kStageRegs));
+        const unsigned st = threadIdx.x - kComputeThreads;
+        unsigned k = 0;
+        bool ok = true;
+        for (unsigned w = blockIdx.x; w < items; w += gridDim.x, ++k) {
+            const unsigned b = k % NB;
+            const QaoaInst I = P.inst[w >> P.li];
+            if (k >= NB && !mb_wait(empty + b, (k / NB - 1) & 1u, P.wait_limit)) { ok = false; break; }
+            if (st == 0) {
+                *reinterpret_cast<QaoaItem*>(smem_q + L.item + kQaoaItemBytes * b) = qaoa_item(P, T, I, w, sizeof(CostT));
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                if (P.layer_a >= 0 && P.kind == kQaoaLow) mb_expect(full + b, 16u << C);
+            }
+            if (kBytes && P.layer_phase >= 0) {
+                const double2* row = T.phase + ((idx_t)I.pos * P.p + P.layer_phase) * T.tstride;
+                double2* tab = reinterpret_cast<double2*>(smem_q + L.tab + L.tab_stride * b);
+                for (unsigned e = st; e < T.tstride; e += kStageThreads)
+                    QaoaDevPsi{const_cast<double2*>(row)}.cp16(tab + e, e);
+            }
+            if (P.layer_a >= 0)
+                qaoa_fill(P.geo, QaoaDevPsi{I.psi}, w & ((1u << P.li) - 1), reinterpret_cast<double2*>(smem_q + L.buf_stride * b),
+                          full + b, st, kStageThreads);
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(sm_u32(full + b)) : "memory");
+            if (st == 0) mb_arrive(full + b);
+        }
+        if (!ok) *P.status = 1.0;
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        // the bulk copies land before the block's shared memory is given up: their items are
+        // computed first, except after an error
+        if (!ok)
+            for (unsigned b = 0; b < NB && b < k; ++b)
+                mb_wait(full + b, ((k - 1 - b) / NB) & 1u, P.wait_limit);
+        return;
+    }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kComputeRegs));
+    const unsigned gid = warp / (GT / 32), tid = threadIdx.x % GT;
+    double* red = reinterpret_cast<double*>(smem_q + L.red) + gid * (GT / 32);
+    auto group_sync = [&] { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + gid), "n"(GT) : "memory"); };
+    unsigned k = gid;
+    for (unsigned w = blockIdx.x + gid * gridDim.x; w < items; w += NG * gridDim.x, k += NG) {
+        const unsigned b = k % NB, parity = (k / NB) & 1u;
+        unsigned char* flag = flags + 2 * gid + ((k / NG) & 1u);
+        if (tid == 0) *flag = mb_wait(full + b, parity, P.wait_limit) ? 1 : 0;
+        group_sync();
+        if (!*flag || !mb_wait(full + b, parity, P.wait_limit)) {
+            if (tid == 0) *P.status = 1.0;
+            break;
+        }
+        const QaoaItem& J = *reinterpret_cast<const QaoaItem*>(smem_q + L.item + kQaoaItemBytes * b);
+        double2* vb = reinterpret_cast<double2*>(smem_q + L.buf_stride * b);
+        const double2* tab = reinterpret_cast<const double2*>(smem_q + L.tab + L.tab_stride * b);
+        auto release = [&] {
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mb_arrive(empty + b);
+        };
+        double acc = 0.0;
+        for (unsigned r = 0; r < P.nreg; ++r) {
+            acc = qaoa_stage<CostT>(P, r, J, QaoaDevPsi{J.psi}, QaoaDevCost<CostT>{static_cast<const CostT*>(J.cost)},
+                                    vb, tab, C, tid, GT, release);
+            if (r + 1 < P.nreg) {
+                if (P.stage[r].warp_sync) __syncwarp();
+                else group_sync();
+            }
+        }
+        if (P.layer_phase < 0) {                       // the item's share of the mean, in fixed order
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+            if (lane == 0) red[tid / 32] = acc;
+            group_sync();
+            if (tid == 0) {
+                double s = 0.0;
+                for (unsigned i = 0; i < GT / 32; ++i) s += red[i];
+                P.partial[w] = s;
+            }
+            group_sync();                              // red is read before the next item writes it
+        }
+    }
+}
+
+// Full items: one block per instance holds all 2^n amplitudes and runs the whole circuit.
+template <class CostT>
+__global__ void __launch_bounds__(512, 1) k_qaoa_full(const __grid_constant__ QaoaPass P, const QaoaTables T) {
+    extern __shared__ __align__(128) unsigned char smem_q[];
+    __shared__ double red[16];
+    double2* vb = reinterpret_cast<double2*>(smem_q);
+    const QaoaInst I = P.inst[blockIdx.x];
+    const unsigned nst = qaoa_full_stages(P.geo.m, P.p);
+    double acc = 0.0;
+    for (unsigned r = 0; r < nst; ++r) {
+        acc = qaoa_full_stage<CostT>(P, T, I.pos, I.n, r, QaoaDevCost<CostT>{static_cast<const CostT*>(I.cost)}, vb,
+                                     threadIdx.x, blockDim.x);
+        if (r + 1 < nst) __syncthreads();
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (unsigned i = 0; i < blockDim.x / 32; ++i) s += red[i];
+        P.partial[blockIdx.x] = s;
+    }
+}
+
+// out[pos] = sum of the instance's partials (a fixed share per thread, then a fixed tree) times
+// the factor of its last layer.  One thread per instance took 212 us for the 4096 partials of a
+// 24-qubit instance; one block takes a few.
+constexpr unsigned kFoldThreads = 128;
+__global__ void __launch_bounds__(kFoldThreads) k_qaoa_fold(const QaoaInst* inst, unsigned ninst,
+                                                            const double* partial, idx_t items, const QaoaRx* rx,
+                                                            unsigned p, double* out) {
+    __shared__ double sh[kFoldThreads];
+    const unsigned i = blockIdx.x;
     const idx_t a = inst[i].item0, b = (i + 1 < ninst) ? inst[i + 1].item0 : items;
     double s = 0.0;
-    for (idx_t w = a; w < b; ++w) s += partial[w];
-    out[inst[i].pos] = s;
+    for (idx_t w = a + threadIdx.x; w < b; w += kFoldThreads) s += partial[w];
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    for (unsigned o = kFoldThreads / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[inst[i].pos] = sh[0] * rx[(idx_t)inst[i].pos * p + p - 1].fm;
 }
 
 int sm_count() {
@@ -133,56 +319,42 @@ int sm_count() {
     return v > 0 ? v : 148;
 }
 
-// The launch shape of a pass: shared bytes, ring depth, and the blocks (every item gets a
-// block, up to the resident blocks of all SMs).  Called before any graph capture: it sets
-// the kernels' shared-memory attribute.
-template <unsigned NT, class CostT, unsigned RING>
-int pass_grid(size_t smem, idx_t items, unsigned* grid) {
-    static bool attr = false;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(k_qaoa_pass<NT, CostT, RING>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return (int)e;
-        attr = true;
+constexpr unsigned kQaoaMinC = 11;      // smallest chunk of the pass kernel
+
+// Dynamic shared memory of a pass or full launch.
+size_t pass_smem(unsigned kind, unsigned C, bool bytes, unsigned tstride) {
+    if (kind == kQaoaFull) return size_t(16) << C;
+    const unsigned nb = C >= 13 ? 1u : C == 12 ? 3u : 6u;
+    return qaoa_smem(C, nb, bytes ? tstride : 0u, 512).total;
+}
+
+template <class K>
+int allow_smem(K kern, int regs = 0) {
+    if (regs) {                                        // the register split counts on the launch's registers
+        cudaFuncAttributes fa;
+        const int rc = (int)cudaFuncGetAttributes(&fa, kern);
+        if (rc) return rc;
+        if (fa.numRegs != regs) return (int)cudaErrorInvalidConfiguration;
     }
-    int per = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_qaoa_pass<NT, CostT, RING>, NT, smem);
-    if (e != cudaSuccess) return (int)e;
-    if (per < 1) return (int)cudaErrorInvalidConfiguration;
-    const idx_t cap = (idx_t)sm_count() * per;
-    *grid = (unsigned)(items < cap ? items : cap);
+    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+}
+// Sets the kernels' shared-memory limits on the current device (before any graph capture).
+int prepare_kernels() {
+    int rc;
+    if ((rc = allow_smem(k_qaoa_pass<uint8_t, 11>, kLaunchRegs)) || (rc = allow_smem(k_qaoa_pass<uint8_t, 12>, kLaunchRegs)) ||
+        (rc = allow_smem(k_qaoa_pass<uint8_t, 13>, kLaunchRegs)) || (rc = allow_smem(k_qaoa_pass<double, 11>, kLaunchRegs)) ||
+        (rc = allow_smem(k_qaoa_pass<double, 12>, kLaunchRegs)) || (rc = allow_smem(k_qaoa_pass<double, 13>, kLaunchRegs)) ||
+        (rc = allow_smem(k_qaoa_full<uint8_t>)) || (rc = allow_smem(k_qaoa_full<double>)))
+        return rc;
     return 0;
 }
 
-constexpr size_t kSmemLimit = 227 * 1024;
-
-template <unsigned NT, class CostT>
-int pass_grid_n(unsigned ring, size_t smem, idx_t items, unsigned* grid) {
-    return ring == 2 ? pass_grid<NT, CostT, 2>(smem, items, grid) : pass_grid<NT, CostT, 1>(smem, items, grid);
-}
-
 template <class CostT>
-int pass_grid_t(unsigned nt, unsigned ring, unsigned lc, idx_t items, unsigned* grid) {
-    const size_t smem = qaoa_smem_bytes<CostT>(lc, nt, ring);
-    if (smem > kSmemLimit) return (int)cudaErrorInvalidConfiguration;
-    if (nt == 128) return pass_grid_n<128, CostT>(ring, smem, items, grid);
-    if (nt == 256) return pass_grid_n<256, CostT>(ring, smem, items, grid);
-    return pass_grid_n<512, CostT>(ring, smem, items, grid);
-}
-
-template <unsigned NT, class CostT>
-void launch_n(unsigned ring, unsigned grid, size_t smem, const QaoaPass& P, const QaoaTables& T, cudaStream_t st) {
-    if (ring == 2) k_qaoa_pass<NT, CostT, 2><<<grid, NT, smem, st>>>(P, T);
-    else k_qaoa_pass<NT, CostT, 1><<<grid, NT, smem, st>>>(P, T);
-}
-
-template <class CostT>
-int launch_pass_t(unsigned nt, unsigned ring, unsigned lc, unsigned grid, const QaoaPass& P, const QaoaTables& T,
-                  cudaStream_t st) {
-    const size_t smem = qaoa_smem_bytes<CostT>(lc, nt, ring);
-    if (nt == 128) launch_n<128, CostT>(ring, grid, smem, P, T, st);
-    else if (nt == 256) launch_n<256, CostT>(ring, grid, smem, P, T, st);
-    else launch_n<512, CostT>(ring, grid, smem, P, T, st);
+int launch_pass_t(unsigned nt, unsigned grid, size_t smem, const QaoaPass& P, const QaoaTables& T, cudaStream_t st) {
+    if (P.kind == kQaoaFull) k_qaoa_full<CostT><<<grid, nt, smem, st>>>(P, T);
+    else if (P.C == 11) k_qaoa_pass<CostT, 11><<<grid, PassShape<11>::kBlock, smem, st>>>(P, T);
+    else if (P.C == 12) k_qaoa_pass<CostT, 12><<<grid, PassShape<12>::kBlock, smem, st>>>(P, T);
+    else k_qaoa_pass<CostT, 13><<<grid, PassShape<13>::kBlock, smem, st>>>(P, T);
     return (int)cudaGetLastError();
 }
 
@@ -196,18 +368,22 @@ struct Graph {                     // one distinct cost function
     std::vector<unsigned char> edges;
     std::vector<double> w;
     unsigned cmax;                 // byte costs: integer maximum; else 0xffffffff
-    void* d_cost = nullptr;
-    uint8_t* d_cost_t = nullptr;   // byte costs: transposed for high passes of chunks of 2^cost_t_C
-    unsigned cost_t_C = 0;         // 0: not filled yet
+    // 2^n costs: those of the low and of the high passes (2^(n-1) each), or of the full pass
+    unsigned char* d_cost = nullptr;
+    size_t cost_bytes = 0;         // of one cost
+    unsigned cost_C = 0;           // chunk size they are ordered for (0: not filled yet)
+    QaoaEdges dev{};               // edges and weights on the device
+    void* high() const { return d_cost + (cost_bytes << (n - 1)); }
 };
 
 struct Launch {
     int what;                      // 0 pass, 1 fold
     unsigned inst_off, ninst;      // slice of the plan's instance records
     idx_t items;
-    unsigned pass, C, kind, nt, ring;
+    unsigned pass, C, kind, nt;
     unsigned n;                    // qubit count of every instance of the launch
     unsigned grid;                 // blocks (pass launches)
+    size_t smem;                   // dynamic shared memory of a block (pass launches)
     bool bytes;                    // byte costs
     size_t partial_off;
 };
@@ -237,7 +413,10 @@ struct orkan_qaoa {
     double* d_gamma = nullptr;          // [instance][p]
     QaoaRx* d_rx = nullptr;
     double2* d_table = nullptr;         // [instance][p][tstride]
-    double* d_out = nullptr;
+    double* d_out = nullptr;            // means, then the status of the bounded waits
+    unsigned char* d_costs = nullptr;   // every graph's costs
+    unsigned char* d_uv = nullptr;      // every graph's edges and weights
+    double* d_w = nullptr;
     double* d_partial = nullptr;
     unsigned char* d_arena = nullptr;
     size_t arena_bytes = 0, partial_cap = 0;
@@ -262,18 +441,21 @@ int dalloc(T** p, size_t count) {
 unsigned default_C(unsigned n) { return n <= 12 ? n : std::max(12u, (n + 1) / 2); }
 bool is_full(const orkan_qaoa* b, unsigned n) { return n <= b->cfg[n].C; }
 
-// Default: 2^12-amplitude chunks, 256 threads (one 16-amplitude set per thread and stage),
-// one buffer, so that two blocks share an SM; instances up to 12 qubits in one full pass.
-// Measured on 16 instances (p = 4, byte costs): 21.1 ms per run at 24 qubits against 23.4 ms
-// for 2^13 with 512 threads, 9.6 against 11.6 ms at 23 qubits.
-QaoaCfg default_cfg(unsigned n) {
+// The launch shape that goes with a chunk size: threads per item (16 amplitudes each; a full
+// item of fewer amplitudes than that takes one warp at least) and buffers per item in work.
+QaoaCfg cfg_for(unsigned n, unsigned C) {
     QaoaCfg c;
-    c.C = default_C(n);
-    c.nt = c.C >= 13 ? 512u : c.C >= 12 ? 256u : 128u;
-    c.ring = 1;
+    c.C = C;
+    c.nt = C >= 13 ? 512u : C == 12 ? 256u : 128u;
+    c.ring = (C >= 13 || n <= C) ? 1u : 2u;
     return c;
 }
-size_t state_bytes(const orkan_qaoa* b, unsigned n) { return is_full(b, n) ? 0 : (size_t(1) << n) * 16; }
+
+// Default: 2^12-slot chunks, two items in work per block and a third one staged; instances up
+// to 12 qubits in one full pass, 25 and 26 qubits in 2^13-slot chunks (n <= 2 C).  A high pass
+// of up to 20 qubits then mixes 8 bits in two groups (three stages instead of five).
+QaoaCfg default_cfg(unsigned n) { return cfg_for(n, default_C(n)); }
+size_t state_bytes(const orkan_qaoa* b, unsigned n) { return is_full(b, n) ? 0 : (size_t(1) << (n - 1)) * 16; }
 
 // Launch plan for the instances `sel` (qubit counts descending), in waves under the budget.
 Plan make_plan(const orkan_qaoa* b, const std::vector<unsigned>& sel) {
@@ -314,14 +496,13 @@ Plan make_plan(const orkan_qaoa* b, const std::vector<unsigned>& sel) {
                     L.kind = full ? kQaoaFull : ((j % 2 == 0) ? kQaoaLow : kQaoaHigh);
                     L.nt = b->cfg[nq].nt;
                     L.n = nq;
-                    L.ring = b->cfg[nq].ring;
                     L.bytes = bytes_cost;
                     idx_t acc = 0;
                     for (size_t k : grp) {
                         QaoaInst r;
                         r.psi = reinterpret_cast<double2*>(off[k - first]);
                         const Graph& gr = b->graphs[b->gid[sel[k]]];
-                        r.cost = (L.kind == kQaoaHigh && bytes_cost) ? static_cast<const void*>(gr.d_cost_t) : gr.d_cost;
+                        r.cost = L.kind == kQaoaHigh ? gr.high() : gr.d_cost;
                         r.item0 = acc;
                         r.n = nq;
                         r.pos = sel[k];
@@ -347,25 +528,40 @@ Plan make_plan(const orkan_qaoa* b, const std::vector<unsigned>& sel) {
     return pl;
 }
 
-// Device side of a plan: arena, partial sums, the instance records, and the transposed byte
-// costs of the plan's high passes for their chunk size.
+// Fill a graph's costs in the orders of its passes for chunks of 2^C.
+int fill_costs(orkan_qaoa* b, Graph& g, unsigned C) {
+    const bool full = g.n <= C, bytes = g.cost_bytes == 1;
+    const unsigned Cc = full ? g.n : C;
+    for (unsigned kind : {(unsigned)kQaoaFull, (unsigned)kQaoaLow, (unsigned)kQaoaHigh}) {
+        if (full != (kind == kQaoaFull)) continue;
+        const idx_t count = idx_t(1) << (full ? g.n : g.n - 1);
+        const unsigned grid = (unsigned)std::min<idx_t>((count + 255) / 256, (idx_t)sm_count() * 16);
+        void* dst = kind == kQaoaHigh ? g.high() : g.d_cost;
+        const QaoaGeo geo = qaoa_geo(g.n, Cc, kind);
+        if (bytes) k_qaoa_cost<<<grid, 256, 0, b->cap>>>((uint8_t*)dst, geo, count, g.dev);
+        else k_qaoa_cost<<<grid, 256, 0, b->cap>>>((double*)dst, geo, count, g.dev);
+        if (const int rc = (int)cudaGetLastError()) return rc;
+    }
+    g.cost_C = C;
+    return 0;
+}
+
+// Device side of a plan: the costs in the order of its passes, arena, partial sums, launch
+// shapes and the instance records.
 int upload_plan(orkan_qaoa* b, Plan& pl) {
     int rc;
-    bool transposed = false;
+    bool filled = false;
     for (const auto& L : pl.launches) {
-        if (L.what != 0 || L.kind != kQaoaHigh || !L.bytes) continue;
+        if (L.what != 0) continue;
         for (unsigned k = L.inst_off; k < L.inst_off + L.ninst; ++k) {
             Graph& g = b->graphs[b->gid[pl.inst[k].pos]];
-            if (g.cost_t_C == L.C) continue;
-            const idx_t tiles = ((idx_t(1) << (g.n - L.C)) + 31) / 32 * (((idx_t(1) << L.C) + 31) / 32);
-            const unsigned grid = (unsigned)std::min<idx_t>(tiles, (idx_t)sm_count() * 8);
-            k_qaoa_cost_transpose<<<grid, dim3(32, 8), 0, b->cap>>>(g.d_cost_t, (const uint8_t*)g.d_cost, g.n, L.C);
-            if ((rc = (int)cudaGetLastError())) return rc;
-            g.cost_t_C = L.C;
-            transposed = true;
+            const unsigned C = b->cfg[g.n].C;
+            if (g.cost_C == C) continue;
+            if ((rc = fill_costs(b, g, C))) return rc;
+            filled = true;
         }
     }
-    if (transposed && (rc = (int)cudaStreamSynchronize(b->cap))) return rc;
+    if (filled && (rc = (int)cudaStreamSynchronize(b->cap))) return rc;
     if (pl.arena > b->arena_bytes) {
         cudaFree(b->d_arena);
         b->d_arena = nullptr;
@@ -382,9 +578,9 @@ int upload_plan(orkan_qaoa* b, Plan& pl) {
     }
     for (auto& L : pl.launches) {
         if (L.what != 0) continue;
-        rc = L.bytes ? pass_grid_t<uint8_t>(L.nt, L.ring, L.C, L.items, &L.grid)
-                     : pass_grid_t<double>(L.nt, L.ring, L.C, L.items, &L.grid);
-        if (rc) return rc;
+        if (L.items > 0xffffffffull / 4) return (int)cudaErrorInvalidConfiguration;     // 32-bit item counters
+        L.smem = pass_smem(L.kind, L.C, L.bytes, b->tstride);
+        L.grid = L.kind == kQaoaFull ? L.ninst : (unsigned)std::min<idx_t>(L.items, (idx_t)sm_count());
     }
     for (auto& r : pl.inst) r.psi = reinterpret_cast<double2*>(b->d_arena + reinterpret_cast<size_t>(r.psi));
     if (pl.inst.size() > b->inst_cap) {
@@ -414,12 +610,13 @@ int enqueue_kernels(const orkan_qaoa* b, const Plan& pl, cudaStream_t st) {
             P.pass = L.pass;
             P.C = L.C;
             P.kind = L.kind;
+            P.status = b->d_out + b->count;
             qaoa_pass_setup(P, L.n);
-            rc = L.bytes ? launch_pass_t<uint8_t>(L.nt, L.ring, L.C, L.grid, P, T, st)
-                         : launch_pass_t<double>(L.nt, L.ring, L.C, L.grid, P, T, st);
+            rc = L.bytes ? launch_pass_t<uint8_t>(L.nt, L.grid, L.smem, P, T, st)
+                         : launch_pass_t<double>(L.nt, L.grid, L.smem, P, T, st);
         } else {
-            k_qaoa_fold<<<(L.ninst + 127) / 128, 128, 0, st>>>(inst, L.ninst, b->d_partial + L.partial_off, L.items,
-                                                               b->d_out);
+            k_qaoa_fold<<<L.ninst, kFoldThreads, 0, st>>>(inst, L.ninst, b->d_partial + L.partial_off, L.items, b->d_rx,
+                                                          b->p, b->d_out);
             rc = (int)cudaGetLastError();
         }
         if (rc) return rc;
@@ -429,7 +626,7 @@ int enqueue_kernels(const orkan_qaoa* b, const Plan& pl, cudaStream_t st) {
 
 int enqueue_tables(const orkan_qaoa* b, cudaStream_t st) {
     if (!b->any_bytes) return 0;
-    k_qaoa_tables<<<b->count, 128, 0, st>>>(b->d_cmax, b->d_gamma, b->count, b->p, b->tstride, b->d_table);
+    k_qaoa_tables<<<b->count, 128, 0, st>>>(b->d_cmax, b->d_gamma, b->d_rx, b->count, b->p, b->tstride, b->d_table);
     return (int)cudaGetLastError();
 }
 
@@ -441,7 +638,7 @@ int enqueue_run(const orkan_qaoa* b, const Plan& pl, cudaStream_t st) {
     if ((rc = (int)cudaMemcpyAsync(b->d_rx, b->h_rx, np * sizeof(QaoaRx), cudaMemcpyHostToDevice, st))) return rc;
     if ((rc = enqueue_tables(b, st))) return rc;
     if ((rc = enqueue_kernels(b, pl, st))) return rc;
-    return (int)cudaMemcpyAsync(b->h_out, b->d_out, (size_t)b->count * 8, cudaMemcpyDeviceToHost, st);
+    return (int)cudaMemcpyAsync(b->h_out, b->d_out, ((size_t)b->count + 1) * 8, cudaMemcpyDeviceToHost, st);
 }
 
 int rebuild(orkan_qaoa* b) {
@@ -472,19 +669,23 @@ int rebuild(orkan_qaoa* b) {
 // Angles into the pinned staging buffers; rx coefficients with the host's libm, as the
 // per-call rx takes them (cos(theta / 2), sin(theta / 2) with theta = 2 beta).
 void stage_angles(orkan_qaoa* b, const double* gammas, const double* betas) {
-    const size_t np = (size_t)b->count * b->p;
-    for (size_t k = 0; k < np; ++k) {
-        const double theta = 2.0 * betas[k];
-        const unsigned n = b->n[k / b->p];
-        b->h_gamma[k] = gammas[k];
-        b->h_rx[k] = qaoa_rx_coeffs(cos(theta / 2.0), sin(theta / 2.0), n, b->cfg[n].C);
+    double c[64], s[64];
+    for (unsigned i = 0; i < b->count; ++i) {
+        const size_t row = (size_t)i * b->p;
+        for (unsigned k = 0; k < b->p; ++k) {
+            const double theta = 2.0 * betas[row + k];
+            b->h_gamma[row + k] = gammas[row + k];
+            c[k] = cos(theta / 2.0);
+            s[k] = sin(theta / 2.0);
+        }
+        qaoa_rx_coeffs(c, s, b->p, b->n[i], b->cfg[b->n[i]].C, b->h_rx + row);
     }
 }
 
 std::string cache_key(const orkan_qaoa* b, unsigned nq, bool bytes) {
     cudaDeviceProp prop;
     cudaGetDeviceProperties(&prop, b->device);
-    return std::string(prop.name) + "|n" + std::to_string(nq) + "|p" + std::to_string(b->p) + (bytes ? "|u8" : "|f64") + "|v2";
+    return std::string(prop.name) + "|n" + std::to_string(nq) + "|p" + std::to_string(b->p) + (bytes ? "|u8" : "|f64") + "|v3";
 }
 
 }  // namespace
@@ -554,31 +755,30 @@ int orkan_qaoa_create(orkan_qaoa_t** out, unsigned count, const unsigned* n_qubi
         }
     }
     b->tstride = cm_all + 1;
-    for (auto& g : b->graphs) {                             // resident cost vectors
-        const bool bytes = g.cmax != 0xffffffffu;
-        const idx_t dim = idx_t(1) << g.n;
-        unsigned char* d_e = nullptr;
-        double* d_w = nullptr;
-        const size_t cbytes = bytes ? ((dim + 15) / 16) * 16 : dim * 8;     // byte costs: whole 16-byte units
-        if ((rc = (int)cudaMalloc(&g.d_cost, cbytes)) ||
-            (bytes && (rc = (int)cudaMalloc(&g.d_cost_t, cbytes))) || (rc = dalloc(&d_e, g.edges.size())) ||
-            (rc = dalloc(&d_w, g.w.size()))) {
-            cudaFree(d_e);
-            orkan_qaoa_destroy(b);
-            return rc;
+    // resident costs, edges and weights of every graph (costs in whole 256-byte units)
+    size_t cost_total = 0, ne = 0;
+    for (auto& g : b->graphs) {
+        g.cost_bytes = g.cmax != 0xffffffffu ? 1 : 8;
+        cost_total += ((g.cost_bytes << g.n) + 255) & ~size_t(255);
+        ne += g.w.size();
+    }
+    if ((rc = dalloc(&b->d_costs, cost_total)) || (rc = dalloc(&b->d_uv, 2 * ne)) || (rc = dalloc(&b->d_w, ne))) {
+        orkan_qaoa_destroy(b);
+        return rc;
+    }
+    {
+        std::vector<unsigned char> uv;
+        std::vector<double> w;
+        size_t at = 0;
+        for (auto& g : b->graphs) {
+            g.d_cost = b->d_costs + at;
+            at += ((g.cost_bytes << g.n) + 255) & ~size_t(255);
+            g.dev = QaoaEdges{b->d_uv + uv.size(), b->d_w + w.size(), (unsigned)g.w.size()};
+            uv.insert(uv.end(), g.edges.begin(), g.edges.end());
+            w.insert(w.end(), g.w.begin(), g.w.end());
         }
-        if (!g.w.empty()) {
-            cudaMemcpy(d_e, g.edges.data(), g.edges.size(), cudaMemcpyHostToDevice);
-            cudaMemcpy(d_w, g.w.data(), g.w.size() * 8, cudaMemcpyHostToDevice);
-        }
-        const unsigned grid = (unsigned)std::min<idx_t>((dim + 255) / 256, (idx_t)sm_count() * 16);
-        if (bytes) k_qaoa_cost<uint8_t><<<grid, 256>>>((uint8_t*)g.d_cost, g.n, d_e, d_w, (unsigned)g.w.size());
-        else k_qaoa_cost<double><<<grid, 256>>>((double*)g.d_cost, g.n, d_e, d_w, (unsigned)g.w.size());
-        rc = (int)cudaGetLastError();
-        if (!rc) rc = (int)cudaDeviceSynchronize();
-        cudaFree(d_e);
-        cudaFree(d_w);
-        if (rc) {
+        if (ne && ((rc = (int)cudaMemcpy(b->d_uv, uv.data(), uv.size(), cudaMemcpyHostToDevice)) ||
+                   (rc = (int)cudaMemcpy(b->d_w, w.data(), w.size() * 8, cudaMemcpyHostToDevice)))) {
             orkan_qaoa_destroy(b);
             return rc;
         }
@@ -588,9 +788,10 @@ int orkan_qaoa_create(orkan_qaoa_t** out, unsigned count, const unsigned* n_qubi
     b->budget = mem_budget ? mem_budget : (unsigned long long)(0.6 * (double)freeb);
     const size_t np = (size_t)count * p;
     if ((rc = dalloc(&b->d_cmax, count)) || (rc = dalloc(&b->d_gamma, np)) || (rc = dalloc(&b->d_rx, np)) ||
-        (rc = dalloc(&b->d_table, b->any_bytes ? np * b->tstride : 1)) || (rc = dalloc(&b->d_out, count)) ||
+        (rc = dalloc(&b->d_table, b->any_bytes ? np * b->tstride : 1)) || (rc = dalloc(&b->d_out, (size_t)count + 1)) ||
         (rc = (int)cudaMallocHost(&b->h_gamma, np * 8)) || (rc = (int)cudaMallocHost(&b->h_rx, np * sizeof(QaoaRx))) ||
-        (rc = (int)cudaMallocHost(&b->h_out, (size_t)count * 8)) ||
+        (rc = (int)cudaMallocHost(&b->h_out, ((size_t)count + 1) * 8)) ||
+        (rc = (int)cudaMemset(b->d_out, 0, ((size_t)count + 1) * 8)) || (rc = prepare_kernels()) ||
         (rc = (int)cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking))) {
         orkan_qaoa_destroy(b);
         return rc;
@@ -614,6 +815,7 @@ int orkan_qaoa_run(orkan_qaoa_t* b, const double* gammas, const double* betas, d
     stage_angles(b, gammas, betas);
     if ((rc = (int)cudaGraphLaunch(b->exec, st))) return rc;
     if ((rc = (int)cudaStreamSynchronize(st))) return rc;
+    if (b->h_out[b->count] != 0.0) return (int)cudaErrorLaunchTimeout;     // a wait for staged data ran out
     memcpy(means, b->h_out, (size_t)b->count * 8);
     return 0;
 }
@@ -637,10 +839,19 @@ int orkan_qaoa_cost_vector(orkan_qaoa_t* b, unsigned i, double* host_out) {
     if (!b || !host_out || i >= b->count) return (int)cudaErrorInvalidValue;
     const Graph& g = b->graphs[b->gid[i]];
     const idx_t dim = idx_t(1) << g.n;
-    if (g.cmax == 0xffffffffu) return (int)cudaMemcpy(host_out, g.d_cost, dim * 8, cudaMemcpyDeviceToHost);
-    std::vector<uint8_t> tmp(dim);
-    const int rc = (int)cudaMemcpy(tmp.data(), g.d_cost, dim, cudaMemcpyDeviceToHost);
-    for (idx_t x = 0; x < dim; ++x) host_out[x] = tmp[x];
+    const bool full = g.n <= g.cost_C;
+    const QaoaGeo geo = qaoa_geo(g.n, full ? g.n : g.cost_C, full ? kQaoaFull : kQaoaLow);
+    double* out = nullptr;
+    int rc = dalloc(&out, dim);
+    if (rc) return rc;
+    const idx_t count = full ? dim : dim / 2;
+    const unsigned grid = (unsigned)std::min<idx_t>((count + 255) / 256, (idx_t)sm_count() * 16);
+    if (g.cost_bytes == 1) k_qaoa_cost_vector<<<grid, 256, 0, b->cap>>>((const uint8_t*)g.d_cost, geo, count, out);
+    else k_qaoa_cost_vector<<<grid, 256, 0, b->cap>>>((const double*)g.d_cost, geo, count, out);
+    rc = (int)cudaGetLastError();
+    if (!rc) rc = (int)cudaStreamSynchronize(b->cap);
+    if (!rc) rc = (int)cudaMemcpy(host_out, out, dim * 8, cudaMemcpyDeviceToHost);
+    cudaFree(out);
     return rc;
 }
 
@@ -678,9 +889,8 @@ int orkan_qaoa_tune(orkan_qaoa_t* b, const double* gammas, const double* betas, 
         if (at != std::string::npos &&
             sscanf(cached.c_str() + at + key.size() + 2, ": {\"C\": %u, \"threads\": %u, \"ring\": %u", &c.C, &c.nt,
                    &c.ring) == 3 &&
-            c.C <= kQaoaMaxC && (c.C >= nq || 2 * c.C >= nq) && (c.nt == 128 || c.nt == 256 || c.nt == 512) &&
-            (c.ring == 1 || c.ring == 2)) {
-            b->cfg[nq] = c;
+            c.C <= kQaoaMaxC && (c.C >= nq || (2 * c.C >= nq && c.C >= kQaoaMinC))) {
+            b->cfg[nq] = cfg_for(nq, c.C);
             continue;
         }
         // up to 64 instances of the group, within one wave's budget
@@ -688,25 +898,16 @@ int orkan_qaoa_tune(orkan_qaoa_t* b, const double* gammas, const double* betas, 
         size_t bytes = 0;
         for (unsigned i = 0; i < b->count && sel.size() < 64; ++i)
             if (b->n[i] == nq && (b->cmax[i] < kQaoaMaxTable) == grp.second) {
-                if (!sel.empty() && bytes + (size_t(1) << nq) * 16 > b->budget) break;
-                bytes += (size_t(1) << nq) * 16;
+                if (!sel.empty() && bytes + (size_t(1) << (nq - 1)) * 16 > b->budget) break;
+                bytes += (size_t(1) << (nq - 1)) * 16;
                 sel.push_back(i);
             }
         // candidates: chunks from the smallest that keeps the high pass possible (2C >= n)
-        // up to 2^13 (a chunk of at least n qubits is the full pass, where only n matters),
-        // thread counts that give a register stage 1..4 sets per thread, ring depth 1 or 2
+        // up to 2^13 (a chunk of at least n qubits is the full pass, where only n matters)
         std::vector<QaoaCfg> cands;
-        const unsigned c_lo = std::min(kQaoaMaxC, std::max(nq <= 11 ? nq : 11u, (nq + 1) / 2));
+        const unsigned c_lo = std::min(kQaoaMaxC, std::max(nq <= kQaoaMinC ? nq : kQaoaMinC, (nq + 1) / 2));
         for (unsigned Cc = c_lo; Cc <= kQaoaMaxC; ++Cc) {
-            const unsigned lc = Cc >= nq ? nq : Cc;
-            for (unsigned tt : {128u, 256u, 512u}) {
-                const unsigned sets = (1u << lc) / 16;       // 16-amplitude sets of a register stage
-                if (tt > std::max(128u, sets) || tt * 4 < sets) continue;
-                for (unsigned rg : {1u, 2u}) {
-                    const size_t smem = grp.second ? qaoa_smem_bytes<uint8_t>(lc, tt, rg) : qaoa_smem_bytes<double>(lc, tt, rg);
-                    if (smem <= kSmemLimit) cands.push_back(QaoaCfg{Cc, tt, rg});
-                }
-            }
+            cands.push_back(cfg_for(nq, Cc));
             if (Cc >= nq) break;                            // a full pass: larger chunks change nothing
         }
         // three rounds over the candidates, interleaved, each timing three runs of the
@@ -782,10 +983,9 @@ void orkan_qaoa_destroy(orkan_qaoa_t* b) {
     if (!b) return;
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->cap) cudaStreamDestroy(b->cap);
-    for (auto& g : b->graphs) {
-        cudaFree(g.d_cost);
-        cudaFree(g.d_cost_t);
-    }
+    cudaFree(b->d_costs);
+    cudaFree(b->d_uv);
+    cudaFree(b->d_w);
     cudaFree(b->d_cmax);
     cudaFree(b->d_gamma);
     cudaFree(b->d_rx);

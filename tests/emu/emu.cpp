@@ -85,21 +85,23 @@ struct EmuMemC2 {
     }
 };
 
-// Cost vector accessor of the QAOA fill: the FP64 cost of amplitude i, or runs of byte
-// costs (len counts the allocated bytes, whole 16-byte units).
+// Cost accessor of the QAOA stages: the FP64 or byte cost i of an item whose costs start at
+// base, or the 2^K byte costs at i (a multiple of 2^K) as words.
 template <class CostT>
 struct EmuCost {
     const CostT* p;
-    idx_t len;
+    idx_t base, len;
     uint64_t* oob;
-    void cpw(double* dst, idx_t i) const {
-        if (i >= len) { ++*oob; return; }
-        *dst = (double)p[i];
+    CostT ld(idx_t i) const {
+        if (base + i >= len) { ++*oob; return CostT(0); }
+        return p[base + i];
     }
-    // byte costs: `bytes` costs from i (a multiple of bytes), within the allocated bytes
-    void cpb(uint8_t* dst, idx_t i, unsigned bytes) const {
-        if ((bytes != 4 && bytes != 8 && bytes != 16) || i % bytes || i + bytes > len) { ++*oob; return; }
-        memcpy(dst, reinterpret_cast<const uint8_t*>(p) + i, bytes);
+    template <int K>
+    void words(uint32_t* w, idx_t i) const {
+        const idx_t nb = idx_t(1) << K;
+        if ((base + i) % nb || base + i + nb > len) { ++*oob; return; }
+        w[0] = 0;
+        memcpy(w, reinterpret_cast<const uint8_t*>(p) + base + i, nb);
     }
 };
 
@@ -170,19 +172,25 @@ void run_phase(int layout, unsigned log_tile, const EmuMem& mem, unsigned n, con
 
 
 // One instance through the fused QAOA passes 0..upto (the GPU launch plan with a single
-// instance): full pass when n <= C, else p + 1 low/high passes of 2^C-amplitude chunks.
+// instance): full pass when n <= C, else p + 1 low/high passes of 2^C-slot items over the
+// stored half of the state.  psi, reads and writes are given for all 2^n basis states: each
+// gets what its stored image holds.
 template <class CostT>
 int run_qaoa(unsigned n, const CostT* cost, unsigned p, const double* gamma, const double* beta, unsigned C,
              unsigned nthr, unsigned upto, double* psi, double* mean, uint32_t* reads, uint32_t* writes,
              uint64_t* oob) {
     const bool full = n <= C;
     if (p == 0 || nthr % 32 || (!full && 2 * C < n) || C > kQaoaMaxC) return -1;
-    const idx_t dim = idx_t(1) << n;
+    const idx_t dim = idx_t(1) << n, half = full ? 0 : dim / 2;
+    std::vector<double> co(p), si(p);
+    for (unsigned k = 0; k < p; ++k) {
+        co[k] = cos(2.0 * beta[k] / 2.0);
+        si[k] = sin(2.0 * beta[k] / 2.0);
+    }
     std::vector<QaoaRx> rx(p);
+    qaoa_rx_coeffs(co.data(), si.data(), p, n, C, rx.data());
     std::vector<double2> table(1, c2(1.0, 0.0));
     unsigned tstride = 1;
-    for (unsigned k = 0; k < p; ++k)
-        rx[k] = qaoa_rx_coeffs(cos(2.0 * beta[k] / 2.0), sin(2.0 * beta[k] / 2.0), n, C);
     if (sizeof(CostT) == 1) {
         unsigned cmax = 0;
         for (idx_t x = 0; x < dim; ++x) cmax = cost[x] > cmax ? (unsigned)cost[x] : cmax;
@@ -192,26 +200,17 @@ int run_qaoa(unsigned n, const CostT* cost, unsigned p, const double* gamma, con
             for (unsigned c = 0; c <= cmax; ++c) {
                 double sn, cs;
                 sincos((double)c * gamma[k], &sn, &cs);
-                table[(size_t)k * tstride + c] = c2(cs, sn);
+                table[(size_t)k * tstride + c] = c2(cs * rx[k].fs, sn * rx[k].fs);
             }
     }
+    std::vector<double2> st((size_t)half);
+    std::vector<uint32_t> rd((size_t)half), wr((size_t)half);
+    const EmuMem mem{st.data(), half, rd.data(), wr.data(), oob};
     QaoaInst I;
-    I.psi = reinterpret_cast<double2*>(psi);
-    I.cost = cost;
+    I.psi = st.data();
     I.item0 = 0;
     I.n = n;
     I.pos = 0;
-    const EmuMem mem{reinterpret_cast<double2*>(psi), dim, reads, writes, oob};
-    const idx_t clen = sizeof(CostT) == 1 ? ((dim + 15) / 16) * 16 : dim;
-    const EmuCost<CostT> cmem{cost, clen, oob};
-    // byte costs of the high passes: the transposed array (qaoa_cost_t_index), as the batch
-    // context builds it for the chunk size
-    std::vector<CostT> cost_t;
-    if (sizeof(CostT) == 1 && !full) {
-        cost_t.assign((size_t)clen, CostT(0));
-        for (idx_t x = 0; x < dim; ++x) cost_t[(size_t)qaoa_cost_t_index(n, C, x)] = cost[x];
-    }
-    const EmuCost<CostT> cmem_t{cost_t.empty() ? cost : cost_t.data(), clen, oob};
     const unsigned npass = full ? 1 : p + 1;
     for (unsigned j = 0; j < npass && j <= upto; ++j) {
         QaoaPass P;
@@ -221,30 +220,53 @@ int run_qaoa(unsigned n, const CostT* cost, unsigned p, const double* gamma, con
         P.C = full ? n : C;
         P.items = qaoa_items(n, P.C, P.kind);
         P.gamma = gamma;
-        std::vector<double> partial(P.items, 0.0);
-        P.partial = partial.data();
         P.p = p;
         P.pass = full ? 0 : j;
         qaoa_pass_setup(P, n);
         const QaoaTables T{table.data(), rx.data(), tstride};
-        const QaoaPlan& pl = P.plan;
-        std::vector<unsigned char> smem(qaoa_smem_bytes<CostT>(P.C, nthr, 1));
-        const QaoaSmem<CostT> S = qaoa_smem_at<CostT>(smem.data(), P.C, nthr, 1, 0);
-        const bool transposed = P.kind == kQaoaHigh && !cost_t.empty();
-        I.cost = transposed ? static_cast<const void*>(cost_t.data()) : static_cast<const void*>(cost);
-        const EmuCost<CostT>& cm = transposed ? cmem_t : cmem;
+        // the costs in the order of the pass, as the batch context makes them
+        const idx_t ncost = full ? dim : half;
+        std::vector<CostT> ordered((size_t)ncost);
+        for (idx_t i = 0; i < ncost; ++i) ordered[(size_t)i] = cost[qaoa_cost_state(P.geo, sizeof(CostT) == 1, i)];
+        I.cost = ordered.data();
+        const unsigned lc = qaoa_lc(n, P.C, P.kind);
+        std::vector<double2> vb((size_t)1 << lc);
+        double sum = 0.0;
         for (idx_t w = 0; w < P.items; ++w) {
-            for (unsigned t = 0; t < nthr; ++t) qaoa_fill<CostT>(P, T, I, pl, mem, cm, w, S, t, nthr);
-            for (unsigned st = 0; st < qaoa_stages(pl); ++st)
-                for (unsigned t = 0; t < nthr; ++t) qaoa_stage<CostT>(P, T, I, pl, mem, w, st, S, t, nthr);
+            std::vector<double> acc(nthr, 0.0);
+            const EmuCost<CostT> cm{ordered.data(), full ? 0 : w << P.C, ncost, oob};
+            if (full) {
+                for (unsigned r = 0; r < qaoa_full_stages(P.geo.m, p); ++r)
+                    for (unsigned t = 0; t < nthr; ++t)
+                        acc[t] = qaoa_full_stage<CostT>(P, T, 0, n, r, cm, vb.data(), t, nthr);
+            } else {
+                const QaoaItem J = qaoa_item(P, T, I, w, sizeof(CostT));
+                if (P.layer_a >= 0)
+                    for (unsigned t = 0; t < nthr; ++t) qaoa_fill(P.geo, mem, J.item, vb.data(), nullptr, t, nthr);
+                for (unsigned r = 0; r < P.nreg; ++r)
+                    for (unsigned t = 0; t < nthr; ++t)
+                        acc[t] = qaoa_stage<CostT>(P, r, J, mem, cm, vb.data(), table.data() + (P.layer_phase < 0 ? 0 : P.layer_phase) * tstride,
+                                                   lc, t, nthr, QaoaNoRelease{});
+            }
+            for (unsigned t = 0; t < nthr; ++t) sum += acc[t];
         }
-        if (pl.measure) {
-            double s = 0.0;
-            for (idx_t w = 0; w < P.items; ++w) s += partial[w];
-            *mean = s;
-        }
+        if (full || j == p) *mean = sum * rx[p - 1].fm;
     }
+    if (!full)
+        for (idx_t x = 0; x < dim; ++x) {
+            const idx_t i = qaoa_index_of(n, C, x);
+            reinterpret_cast<double2*>(psi)[x] = st[(size_t)i];
+            reads[x] = rd[(size_t)i];
+            writes[x] = wr[(size_t)i];
+        }
     return 0;
+}
+
+// Slots that thread t of nthr touches in group gi of a chunked item, marked with its half-warp.
+template <int K, int B0>
+void mark_s(const QaoaGeo& g, std::vector<unsigned>& own) {
+    for (unsigned r = 0; r < (1u << (g.C - K)); ++r)
+        for (unsigned e = 0; e < (1u << K); ++e) own[qaoa_s_base<K, B0>(g.MM, r) + (e << B0)] = r >> 4;
 }
 
 }  // namespace
@@ -466,13 +488,30 @@ int emu_fused_stages(unsigned n, unsigned log_chunk, unsigned ngates, const orka
     return (int)P.nstages;
 }
 
-// Shared-memory layout of the QAOA pass kernel: 1 when every region is aligned for all
-// chunk sizes 0..13 and ring depths 1, 2, for both cost types.
+// Shared-memory layout of the QAOA pass kernel: 1 when every region is aligned for the chunk
+// sizes and buffer counts of the launches and any table length.
 int emu_qaoa_smem_aligned(void) {
-    for (unsigned C = 0; C <= kQaoaMaxC; ++C)
-        for (unsigned ring = 1; ring <= 2; ++ring)
-            if (!qaoa_smem_aligned<uint8_t>(C, ring) || !qaoa_smem_aligned<double>(C, ring)) return 0;
+    for (unsigned C = 1; C <= kQaoaMaxC; ++C)
+        for (unsigned buffers = 1; buffers <= 6; ++buffers)
+            for (unsigned tstride = 0; tstride <= kQaoaMaxTable; ++tstride)
+                if (!qaoa_smem_aligned(C, buffers, tstride, 512)) return 0;
     return 1;
+}
+
+// Groups 0 and 1 of a pass's items, when both hold 16 amplitudes: 1 when every half-warp
+// touches the same slots in both, every slot once (0 otherwise, -1: not such a pass).
+int emu_qaoa_half_warp_closed(unsigned n, unsigned C, unsigned kind) {
+    const QaoaGeo g = qaoa_geo(n, C, kind);
+    if (g.m < 2 || qaoa_group_bits(g, 0) != 4 || qaoa_group_bits(g, 1) != 4) return -1;
+    std::vector<unsigned> a((size_t)1 << C, ~0u), b((size_t)1 << C, ~0u);
+    for (unsigned r = 0; r < (1u << (C - 4)); ++r)
+        for (unsigned e = 0; e < 16; ++e) {
+            unsigned& o = a[qaoa_m_slot(qaoa_m_set<4>(g.MM, r), 4, e)];
+            if (o != ~0u) return 0;
+            o = r >> 4;
+        }
+    mark_s<4, 4>(g, b);
+    return a == b ? 1 : 0;
 }
 
 // Fused QAOA passes of one instance; byte_cost selects byte costs (cost_b) over doubles.
