@@ -37,6 +37,10 @@ int orkan_mlp_set_params(orkan_mlp_t *m, const float *host);      /* also resets
 /* y_dev[b] = f(x_dev[b][:]) for b < batch. */
 int orkan_mlp_forward(orkan_mlp_t *m, const float *x_dev, unsigned batch, float *y_dev, void *stream);
 
+/* The same for any count, in pieces of max_batch where the network's size needs scratch for the
+ * activations (256 hidden units and at most 64 inputs need none). */
+int orkan_mlp_predict(orkan_mlp_t *m, const float *x_dev, unsigned count, float *y_dev, void *stream);
+
 /* Loss L = mean_b (f(x_b) - t_b)^2 and its gradients: grad_dev (param_count floats, the
  * parameter-vector layout) and, when gx_dev is not NULL, dL/dx [batch][n_in].  loss_dev
  * receives L (one float).  No parameter changes. */

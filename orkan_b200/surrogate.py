@@ -31,12 +31,13 @@ def _declare(lib):
     lib.orkan_mlp_get_params.argtypes = [P, P]
     lib.orkan_mlp_set_params.argtypes = [P, P]
     lib.orkan_mlp_forward.argtypes = [P, P, C.c_uint, P, P]
+    lib.orkan_mlp_predict.argtypes = [P, P, C.c_uint, P, P]
     lib.orkan_mlp_gradients.argtypes = [P, P, P, C.c_uint, P, P, P, P]
     lib.orkan_mlp_train.argtypes = [P, P, P, C.c_uint, C.c_uint, C.c_uint, C.c_float, C.c_ulonglong, P, P]
     lib.orkan_mlp_ascend.argtypes = [P, P, C.c_uint, C.c_uint, C.c_float, C.c_float, C.c_float, P, P]
     lib.orkan_mlp_launch_count.argtypes = []
     lib.orkan_mlp_launch_count.restype = C.c_ulonglong
-    for f in ("create", "get_params", "set_params", "forward", "gradients", "train", "ascend"):
+    for f in ("create", "get_params", "set_params", "forward", "predict", "gradients", "train", "ascend"):
         getattr(lib, "orkan_mlp_" + f).restype = C.c_int
     lib._mlp_declared = True
 
@@ -84,10 +85,8 @@ class Mlp:
         import torch
         n = x.shape[0]
         y = torch.empty(n, dtype=torch.float32, device=x.device)
-        for c0 in range(0, n, self.max_batch):
-            c1 = min(n, c0 + self.max_batch)
-            xs, ys = x[c0:c1], y[c0:c1]
-            _check(self.lib.orkan_mlp_forward(self.h, _ptr(xs), c1 - c0, _ptr(ys), _stream()), "forward")
+        if n:
+            _check(self.lib.orkan_mlp_predict(self.h, _ptr(x), n, _ptr(y), _stream()), "predict")
         return y
 
     def gradients(self, x, t, want_x=False):
