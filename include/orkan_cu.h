@@ -105,6 +105,12 @@ int orkan_cu_dm_phase(int layout, unsigned log_tile, void *rho, unsigned n, unsi
 int orkan_cu_dm_superop1(int layout, unsigned log_tile, void *rho, unsigned n, unsigned target,
                          const double *sop, void *stream);
 
+/* count 1-qubit channels, channel i with the 4 x 4 superoperator at sops + 32 i (as above) on
+ * targets[i], in the given order: channels on one qubit are multiplied, and chains of up to six
+ * qubits that fit one staged block are applied in one pass over the matrix. */
+int orkan_cu_dm_channels(int layout, unsigned log_tile, void *rho, unsigned n, unsigned count,
+                         const unsigned *targets, const double *sops, void *stream);
+
 /* 2-qubit superoperator on (q0, q1): sop = 16 x 16 row-major complex over vec(rho_4x4) with
  * vec index 4 * row + column and local index 2 * bit(q0) + bit(q1).  No counterpart in the
  * reference, whose channel_1q takes 1-local superoperators only (src/channel/channel.c:67-85)

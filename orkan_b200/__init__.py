@@ -103,6 +103,10 @@ class Orkan:
         L.kraus_to_superop.argtypes = [C.POINTER(KrausT)]
         L.kraus_to_superop.restype = SuperopT
         L.channel_1q.argtypes = [P, C.POINTER(SuperopT), C.c_ubyte]
+        L.channel_1q_layer.argtypes = [P, C.POINTER(SuperopT), C.c_void_p, C.c_uint]
+        L.channel_1q_layer.restype = None
+        L.orkan_cu_fill.argtypes = [C.c_int, C.c_uint, vp, C.c_uint, C.c_double, C.c_double, vp]
+        L.orkan_cu_fill.restype = C.c_int
         L.channel_2q.argtypes = [P, C.POINTER(SuperopT), C.c_ubyte, C.c_ubyte]
         L.single_from_mat.argtypes = [P, C.c_ubyte, vp]
         L.two_from_mat.argtypes = [P, C.c_ubyte, C.c_ubyte, vp]
@@ -220,6 +224,13 @@ class Orkan:
         arr = np.ascontiguousarray(np.asarray(sop).reshape(-1), dtype=np.complex128)
         so = SuperopT(1, arr.ctypes.data)
         self.lib.channel_1q(C.byref(s), C.byref(so), int(q))
+
+    def channel_1q_layer(self, s: StateT, sops, qubits) -> None:
+        """1-qubit channels sops[i] (4 x 4 superoperators, or one for all) on qubits[i], in order."""
+        q = np.ascontiguousarray(qubits, dtype=np.uint8)
+        arr = np.ascontiguousarray(np.broadcast_to(np.asarray(sops).reshape(-1, 16), (len(q), 16)), dtype=np.complex128)
+        so = (SuperopT * len(q))(*[SuperopT(1, arr.ctypes.data + 256 * i) for i in range(len(q))])
+        self.lib.channel_1q_layer(C.byref(s), so, q.ctypes.data, len(q))
 
     def channel_2q(self, s: StateT, sop: np.ndarray, q0: int, q1: int) -> None:
         """2-qubit channel (16 x 16 superoperator, local index 2 bit(q0) + bit(q1))."""

@@ -116,6 +116,44 @@ inline bool dm_geometry(unsigned n, unsigned k, const unsigned* qubits, unsigned
     }
 }
 
+// Geometry of a chain of 1-qubit operations on the k distinct qubits of the ascending list
+// qubits: the largest sub-tile whose block, with the qubits above it as pairing bits (at most
+// 3), stays within 64 x 64.  vbit[j] receives the virtual bit of qubits[j].  False when the
+// qubits do not fit one block.
+inline bool dm_chain_geometry(unsigned n, unsigned k, const unsigned* qubits, unsigned ls_max, DmGeom* g,
+                              unsigned* vbit) {
+    if (k < 1 || k > 6 || n < k || qubits[k - 1] >= n) return false;
+    for (int l = (int)(ls_max < n ? ls_max : n); l >= 0; --l) {
+        const unsigned ls = (unsigned)l;
+        unsigned hq[3], h = 0, above = 0;
+        for (unsigned j = 0; j < k; ++j)
+            if (qubits[j] >= ls) {
+                if (above < 3) hq[above] = qubits[j];
+                ++above;
+            }
+        if (above > 3 || ls + above > 6) continue;
+        h = above;
+        if (h == 0 && ls < n && ls + 1 <= 6) hq[h++] = ls;       // pair the sub-tiles along qubit ls
+        g->d = idx_t(1) << n;
+        g->n = n;
+        g->ls = ls;
+        g->h = h;
+        g->k = 1;
+        for (unsigned a = 0; a < 3; ++a) {
+            g->hb[a] = a < h ? hq[a] - ls : 0;
+            g->vbit[a] = 0;
+        }
+        for (unsigned j = 0, rank = 0; j < k; ++j) vbit[j] = qubits[j] < ls ? qubits[j] : ls + rank++;
+        g->nbase = (g->d >> ls) >> h;
+        g->items = g->nbase * (g->nbase + 1) / 2;
+        g->fixmask = 0;
+        g->fixrows = 0;
+        g->hcmask = 0;
+        return true;
+    }
+    return false;
+}
+
 // Sub-tile classes of position (a, b) of an item.
 enum : int { kSubDirect = 0, kSubDiag = 1, kSubTransposed = 2, kSubSkip = 3 };
 
@@ -540,6 +578,145 @@ struct OpSuper1 {
     }
 };
 
+// One term of a superoperator's row: acc += s x as four FMAs.
+ORKAN_HD void super_fma(double2& acc, double2 s, double2 x) {
+    acc.x = fma(s.x, x.x, acc.x);
+    acc.x = fma(-s.y, x.y, acc.x);
+    acc.y = fma(s.x, x.y, acc.y);
+    acc.y = fma(s.y, x.x, acc.y);
+}
+
+// Up to six 1-qubit superoperators on different qubits of the staged block, in stages of one or
+// two: a stage of two keeps the 16 elements of a 4 x 4 group in registers for both, so shared
+// memory is read and written once per pair of channels and HBM once per chain.
+//
+// Bound (64 x 64 block, six channels): 96 FP64 FMAs per element are 1.5 SM clocks, the 32 bytes
+// of HBM traffic 1.3, three stages in shared memory 0.75.
+constexpr unsigned kChainMax = 6;
+struct OpChain {
+    double2 s[kChainMax][16];
+    unsigned nst;
+    struct Stage {
+        unsigned char two;         // two channels: op[0] on bit b[0], then op[1] on bit b[1]
+        unsigned char op[2], b[2];
+    } st[kChainMax];
+
+    // One channel: 2 x 2 groups (as OpSuper1).
+    ORKAN_HD void one(const DmGeom& g, double2* vb, unsigned tid, unsigned nthr, const double2* sp, unsigned vbq) const {
+        const unsigned P = g.P(), lh = g.ls + g.h - 1;
+        const unsigned groups = 1u << (2 * lh);
+        const bool sw = dm_swap_cols(vbq, lh, tid);
+        for (unsigned t = tid; t < groups; t += nthr) {
+            const unsigned r0 = (unsigned)insert0(t >> lh, vbq), c0 = (unsigned)insert0(t & ((1u << lh) - 1), vbq);
+            const unsigned r1 = r0 | (1u << vbq), c1 = c0 | (1u << vbq);
+            const unsigned ca = sw ? c1 : c0, cb = sw ? c0 : c1;
+            const double2 y0a = vb[r0 * P + ca], y0b = vb[r0 * P + cb];
+            const double2 y1a = vb[r1 * P + ca], y1b = vb[r1 * P + cb];
+            const double2 x[4] = {sw ? y0b : y0a, sw ? y0a : y0b, sw ? y1b : y1a, sw ? y1a : y1b};
+            double2 out[4];
+#pragma unroll
+            for (unsigned m = 0; m < 4; ++m) {
+                double2 acc = c2(0.0, 0.0);
+#pragma unroll
+                for (unsigned j = 0; j < 4; ++j) super_fma(acc, sp[4 * m + j], x[j]);
+                out[m] = acc;
+            }
+            vb[r0 * P + ca] = sw ? out[1] : out[0];
+            vb[r0 * P + cb] = sw ? out[0] : out[1];
+            vb[r1 * P + ca] = sw ? out[3] : out[2];
+            vb[r1 * P + cb] = sw ? out[2] : out[3];
+        }
+    }
+
+    // Two channels on bits ba and bb of 4 x 4 groups.  When ba lies below bit 3 (and bb above), lanes
+    // with bit 2 set take a row's columns with the other value of bit ba first (dm_swap_cols).
+    ORKAN_HD void two(const DmGeom& g, double2* vb, unsigned tid, unsigned nthr, const double2* sa, const double2* sb,
+                      unsigned ba, unsigned bb) const {
+        const unsigned P = g.P(), lq = g.ls + g.h - 2;
+        const unsigned asc[2] = {ba < bb ? ba : bb, ba < bb ? bb : ba};
+        const unsigned groups = 1u << (2 * lq);
+        const bool sw = ba < 3 && lq >= 3 && (tid & 4u);
+        const unsigned fa = 1u << ba, fb = 1u << bb;
+        for (unsigned t = tid; t < groups; t += nthr) {
+            unsigned r = t >> lq, c = t & ((1u << lq) - 1);
+            for (unsigned j = 0; j < 2; ++j) {
+                const unsigned lo = (1u << asc[j]) - 1;
+                r = ((r & ~lo) << 1) | (r & lo);
+                c = ((c & ~lo) << 1) | (c & lo);
+            }
+            double2* base = vb + r * P + c;
+            const unsigned c0 = sw ? fa : 0u, c1 = sw ? 0u : fa;      // columns in the order of access
+            double2 x[16];                                            // [row bb][col bb][row ba][col ba]
+#pragma unroll
+            for (unsigned q = 0; q < 4; ++q) {                        // (row, column) value of bit bb
+                double2* e = base + (q >> 1) * fb * P + (q & 1) * fb;
+                const double2 y0a = e[c0], y0b = e[c1], y1a = e[fa * P + c0], y1b = e[fa * P + c1];
+                const double2 y[4] = {sw ? y0b : y0a, sw ? y0a : y0b, sw ? y1b : y1a, sw ? y1a : y1b};
+#pragma unroll
+                for (unsigned m = 0; m < 4; ++m) {
+                    double2 acc = c2(0.0, 0.0);
+#pragma unroll
+                    for (unsigned j = 0; j < 4; ++j) super_fma(acc, sa[4 * m + j], y[j]);
+                    x[4 * q + m] = acc;
+                }
+            }
+#pragma unroll
+            for (unsigned q = 0; q < 2; ++q) {                        // row value of bit ba
+                double2 z[2][4];
+#pragma unroll
+                for (unsigned cc = 0; cc < 2; ++cc)
+#pragma unroll
+                    for (unsigned m = 0; m < 4; ++m) {
+                        double2 acc = c2(0.0, 0.0);
+#pragma unroll
+                        for (unsigned j = 0; j < 4; ++j) super_fma(acc, sb[4 * m + j], x[4 * j + 2 * q + cc]);
+                        z[cc][m] = acc;
+                    }
+#pragma unroll
+                for (unsigned m = 0; m < 4; ++m) {
+                    double2* e = base + (m >> 1) * fb * P + (m & 1) * fb + q * fa * P;
+                    e[c0] = sw ? z[1][m] : z[0][m];
+                    e[c1] = sw ? z[0][m] : z[1][m];
+                }
+            }
+        }
+    }
+
+    // Stage i (a block barrier lies between stages).
+    ORKAN_HD void stage(unsigned i, const DmGeom& g, double2* vb, unsigned tid, unsigned nthr) const {
+        const Stage q = st[i];
+        if (q.two) two(g, vb, tid, nthr, s[q.op[0]], s[q.op[1]], q.b[0], q.b[1]);
+        else one(g, vb, tid, nthr, s[q.op[0]], q.b[0]);
+    }
+    ORKAN_HD void operator()(const DmGeom& g, double2* vb, unsigned tid, unsigned nthr, unsigned = 3u) const {
+        stage(0, g, vb, tid, nthr);                    // whole chains run stage by stage (dm_op_apply)
+    }
+};
+
+// Stages of a chain on virtual bits vbit[0 .. k): a low bit (below 3, where the lanes' order matters)
+// goes with a high one, then the high ones in pairs, then what is left alone.  Channels on different
+// qubits commute.  Operator j acts on vbit[j].
+inline void dm_chain_stages(OpChain& op, unsigned k, const unsigned* vbit) {
+    unsigned lo[kChainMax], hi[kChainMax], nl = 0, nh = 0;
+    for (unsigned j = 0; j < k; ++j) {
+        if (vbit[j] < 3) lo[nl++] = j;
+        else hi[nh++] = j;
+    }
+    op.nst = 0;
+    auto put = [&](unsigned a, unsigned b, bool two) {
+        OpChain::Stage& q = op.st[op.nst++];
+        q.two = two;
+        q.op[0] = (unsigned char)a;
+        q.op[1] = (unsigned char)b;
+        q.b[0] = (unsigned char)vbit[a];
+        q.b[1] = (unsigned char)vbit[b];
+    };
+    while (nl && nh) { --nl; --nh; put(lo[nl], hi[nh], true); }
+    while (nh >= 2) { nh -= 2; put(hi[nh], hi[nh + 1], true); }
+    while (nh) { --nh; put(hi[nh], hi[nh], false); }
+    while (nl) { --nl; put(lo[nl], lo[nl], false); }
+}
+
 // FP64 tensor-core form of the 2-qubit superoperator.  The update of one 4 x 4 group is a real
 // 32 x 32 matrix A (rows: re / im of the 16 outputs; columns: re / im of the 16 inputs) times
 // the group's 32 real inputs; a warp applies it to 8 groups at a time with 4 x 8 steps of
@@ -949,6 +1126,16 @@ inline void dm_orient(OpSuper1& op, bool transposed) {
     for (unsigned i = 0; i < 16; ++i) op.s[i] = t[i];
 }
 
+inline void dm_orient(OpChain& op, bool transposed) {
+    if (!transposed) return;
+    for (auto& m : op.s) {
+        OpSuper1 one;
+        for (unsigned i = 0; i < 16; ++i) one.s[i] = m[i];
+        dm_orient(one, true);
+        for (unsigned i = 0; i < 16; ++i) m[i] = one.s[i];
+    }
+}
+
 // Shared memory of one engine block: the mbarrier, the descriptors, the staged block.
 ORKAN_HD size_t dm_stage_bytes(const DmGeom& g) { return kDmPosBytes + (size_t)g.V() * g.P() * 16; }
 ORKAN_HD size_t dm_block_smem_bytes(const DmGeom& g) { return 16 + dm_stage_bytes(g); }
@@ -1037,6 +1224,14 @@ __device__ __forceinline__ void dm_op_apply(const Op& op, const DmGeom& g, doubl
                                             unsigned iflags, const DmNoThreadState&) {
     op(g, vb, tid, nthr, iflags);
 }
+__device__ __forceinline__ void dm_op_apply(const OpChain& op, const DmGeom& g, double2* vb, unsigned tid,
+                                            unsigned nthr, unsigned, const DmNoThreadState&) {
+#pragma unroll 1
+    for (unsigned i = 0; i < op.nst; ++i) {
+        op.stage(i, g, vb, tid, nthr);
+        if (i + 1 < op.nst) __syncthreads();
+    }
+}
 __device__ __forceinline__ void dm_op_prepare(const OpSuper2& op, const DmGeom& g, Super2Frag& f, double2* vb,
                                               unsigned tid, unsigned nthr) {
     // the same condition for every block of the launch; only the tensor-core form uses the
@@ -1062,6 +1257,7 @@ __device__ __forceinline__ void dm_op_apply(const OpSuper2& op, const DmGeom& g,
 // (64 registers) and gets two.
 template <class Op> struct DmMinBlocks { static constexpr int value = 3; };
 template <> struct DmMinBlocks<OpSuper2> { static constexpr int value = 2; };
+template <> struct DmMinBlocks<OpChain> { static constexpr int value = 2; };   // 16 elements per thread
 
 // Persistent engine: block b handles items b, b + G, b + 2G, ...  One item at a time per
 // block; with up to three blocks resident per SM (71 KB of shared memory each) the bulk

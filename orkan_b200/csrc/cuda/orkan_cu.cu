@@ -368,6 +368,60 @@ int orkan_cu_dm_superop1(int layout, unsigned log_tile, void* rho, unsigned n, u
     return launch_engine_map(layout, log_tile, rho, n, g, op, as_stream(stream));
 }
 
+int orkan_cu_dm_channels(int layout, unsigned log_tile, void* rho, unsigned n, unsigned count, const unsigned* targets,
+                         const double* sops, void* stream) {
+    if (!rho || !targets || !sops || !layout_ok(layout, log_tile) || n < 1 || n > 40) return (int)cudaErrorInvalidValue;
+    for (unsigned i = 0; i < count; ++i)
+        if (targets[i] >= n) return (int)cudaErrorInvalidValue;
+    // channels on different qubits commute; those on one qubit are multiplied in their order
+    double2 s[40][16];
+    bool has[40] = {};
+    for (unsigned i = 0; i < count; ++i) {
+        const unsigned q = targets[i];
+        double2 m[16];
+        for (unsigned e = 0; e < 16; ++e) m[e] = ld_c(sops + 32 * (size_t)i, e);
+        if (!has[q]) {
+            for (unsigned e = 0; e < 16; ++e) s[q][e] = m[e];
+            has[q] = true;
+            continue;
+        }
+        double2 t[16];
+        for (unsigned r = 0; r < 4; ++r)
+            for (unsigned c = 0; c < 4; ++c) {
+                double2 acc = c2(0.0, 0.0);
+                for (unsigned k = 0; k < 4; ++k) super_fma(acc, m[4 * r + k], s[q][4 * k + c]);
+                t[4 * r + c] = acc;
+            }
+        for (unsigned e = 0; e < 16; ++e) s[q][e] = t[e];
+    }
+    unsigned qs[40], k = 0;
+    for (unsigned q = 0; q < n; ++q)
+        if (has[q]) qs[k++] = q;
+    // chains of as many of the lowest remaining qubits as fit one staged block
+    const unsigned ls_max = ls_max_for(layout, log_tile);
+    for (unsigned at = 0; at < k;) {
+        DmGeom g;
+        unsigned vbit[kChainMax], take = k - at < kChainMax ? k - at : kChainMax;
+        while (take > 1 && !dm_chain_geometry(n, take, qs + at, ls_max, &g, vbit)) --take;
+        int rc;
+        if (take == 1) {
+            OpSuper1 op;
+            for (unsigned e = 0; e < 16; ++e) op.s[e] = s[qs[at]][e];
+            if (!dm_geometry(n, 1, qs + at, ls_max, &g, dm_max_v_low())) return (int)cudaErrorInvalidValue;
+            rc = launch_engine_map(layout, log_tile, rho, n, g, op, as_stream(stream));
+        } else {
+            OpChain op;
+            for (unsigned j = 0; j < kChainMax; ++j)
+                for (unsigned e = 0; e < 16; ++e) op.s[j][e] = j < take ? s[qs[at + j]][e] : c2(0.0, 0.0);
+            dm_chain_stages(op, take, vbit);
+            rc = launch_engine_map(layout, log_tile, rho, n, g, op, as_stream(stream));
+        }
+        if (rc) return rc;
+        at += take;
+    }
+    return 0;
+}
+
 int orkan_cu_dm_superop2(int layout, unsigned log_tile, void* rho, unsigned n, unsigned q0, unsigned q1,
                          const double* sop, void* stream) {
     if (!rho || !sop || !layout_ok(layout, log_tile) || q0 >= n || q1 >= n || q0 == q1 || n > 40)

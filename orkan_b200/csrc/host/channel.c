@@ -7,6 +7,8 @@
 #include "channel.h"
 #include "orkan_dev.h"
 
+#include <string.h>
+
 #define CHANNEL_VALIDATE(cond, msg) ORKAN_VALIDATE("channel", cond, msg)
 
 /* S[(i,j),(k,l)] = sum_a K_a[i,k] conj(K_a[j,l]) with row index i*N + j and column
@@ -61,6 +63,32 @@ void channel_1q(state_t *state, const superop_t *sop, const qubit_t target) {
         default:
             CHANNEL_VALIDATE(0, "channel_1q: unknown state type");
     }
+}
+
+/* Several 1-qubit channels in order (extension, include/orkan_dev.h). */
+void channel_1q_layer(state_t *state, const superop_t *sops, const qubit_t *targets, unsigned count) {
+    CHANNEL_VALIDATE(state && state->data, "channel_1q_layer: null state or data pointer");
+    CHANNEL_VALIDATE(count == 0 || (sops && targets), "channel_1q_layer: null superoperators or targets");
+    CHANNEL_VALIDATE(state->type == MIXED_PACKED || state->type == MIXED_TILED,
+                     "channel_1q_layer: not available for pure states");
+    for (unsigned i = 0; i < count; ++i) {
+        CHANNEL_VALIDATE(targets[i] < state->qubits, "channel_1q_layer: target qubit out of range");
+        CHANNEL_VALIDATE(sops[i].data, "channel_1q_layer: null superoperator data pointer");
+        CHANNEL_VALIDATE(sops[i].n_qubits == 1, "channel_1q_layer: superoperator is not 1-local");
+    }
+    if (!count) return;
+    cplx_t *s = (cplx_t *)malloc((size_t)count * 16 * sizeof(cplx_t));
+    unsigned *q = (unsigned *)malloc((size_t)count * sizeof(unsigned));
+    CHANNEL_VALIDATE(s && q, "channel_1q_layer: allocation failed");
+    for (unsigned i = 0; i < count; ++i) {
+        memcpy(s + 16 * (size_t)i, sops[i].data, 16 * sizeof(cplx_t));
+        q[i] = targets[i];
+    }
+    const int rc = orkan_cu_dm_channels((int)state->type, LOG_TILE_DIM, state->data, state->qubits, count, q,
+                                        (const double *)s, orkan_stream());
+    free(s);
+    free(q);
+    orkan_check_cu("channel", "channel_1q_layer", rc);
 }
 
 /* 2-qubit channel (extension, include/orkan_dev.h): the reference's channel_1q accepts

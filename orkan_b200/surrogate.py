@@ -182,40 +182,72 @@ def rx_matrix(theta):
 
 
 class NoisyEvaluator:
-    """Exact FP64 <C> of the noisy circuit on a tiled density matrix through the per-call
-    API: state_plus, then per layer exp_diag(cost, gamma_k) and, on every qubit, rx(2 beta_k)
-    followed by a depolarizing channel -- applied as one channel_1q with the superoperator
-    of the Kraus set {K_i Rx} (kraus_to_superop of the library), then mean(cost)."""
+    """Exact FP64 <C> of the noisy circuit on a density matrix through the per-call API:
+    |+><+|, then per layer exp_diag(cost, gamma_k) and, on every qubit, rx(2 beta_k) followed by a
+    depolarizing channel -- applied as one channel_1q_layer with the superoperator of the Kraus
+    set {K_i Rx} on every qubit -- then mean(cost).  The costs stay on the device, and a state is
+    kept for the next evaluation (one per thread that evaluates at a time, at most four)."""
 
     def __init__(self, ork, n, edges, weights, p, prob, kind="tiled"):
+        import torch
         self.ork, self.n, self.p, self.prob, self.kind = ork, n, p, prob, kind
         x = np.arange(1 << n, dtype=np.int64)
         cost = np.zeros(1 << n)
         for e, (u, v) in enumerate(edges):
             cost += (1.0 if weights is None else float(weights[e])) * (((x >> u) ^ (x >> v)) & 1)
         self.cost = cost
+        self._cost = torch.from_numpy(cost).cuda()
         self.kraus = depolarizing_kraus(prob)
         self.evals = 0
+        self._states = []
 
     def one(self, g, b):
-        ork = self.ork
-        st = ork.plus(self.kind, self.n)
-        for k in range(self.p):
-            ork.exp_diag(st, self.cost, float(g[k]))
-            rx = rx_matrix(2.0 * float(b[k]))
-            sop = ork.superop([K @ rx for K in self.kraus])
-            for q in range(self.n):
-                ork.channel_1q(st, sop, q)
-        m = ork.mean(st, self.cost)
-        ork.free(st)
-        self.evals += 1
-        return m
+        return self._run(np.asarray(g)[None], np.asarray(b)[None])[0]
+
+    def _run(self, gs, bs):
+        ork, n = self.ork, self.n
+        half = np.asarray(bs, dtype=np.float64)
+        rx = np.empty(half.shape + (2, 2), dtype=np.complex128)
+        rx[..., 0, 0] = rx[..., 1, 1] = np.cos(half)
+        rx[..., 0, 1] = rx[..., 1, 0] = -1j * np.sin(half)
+        sops = sum(np.einsum("...ik,...jl->...ijkl", k @ rx, np.conj(k @ rx)) for k in self.kraus)
+        sops = sops.reshape(half.shape + (4, 4))
+        cost, qubits = int(self._cost.data_ptr()), np.arange(n, dtype=np.uint8)
+        try:
+            st = self._states.pop()
+        except IndexError:
+            st = ork.state(self.kind, n)
+        out = np.empty(len(gs))
+        try:
+            for e, g in enumerate(gs):
+                rc = ork.lib.orkan_cu_fill(st.type, ork.log_tile, st.data, n, 1.0 / (1 << n), 0.0,
+                                           ork.lib.orkan_get_stream())
+                if rc:
+                    raise OrkanError(f"fill failed: CUDA error {rc}")
+                for k in range(self.p):
+                    ork.exp_diag(st, cost, float(g[k]))
+                    ork.channel_1q_layer(st, sops[e, k], qubits)
+                out[e] = ork.mean(st, cost)
+        finally:
+            if len(self._states) < 4:
+                self._states.append(st)
+            else:
+                ork.free(st)
+        self.evals += len(gs)
+        return out
 
     def __call__(self, gammas, betas):
-        return np.array([self.one(g, b) for g, b in zip(np.asarray(gammas), np.asarray(betas))])
+        return self._run(np.asarray(gammas), np.asarray(betas))
 
     def close(self):
-        pass
+        while self._states:
+            self.ork.free(self._states.pop())
+
+    def __del__(self):
+        try:
+            self.close()
+        except Exception:
+            pass
 
 
 def plain_sweep(evaluate, p, count, rng, chunk, clock):

@@ -116,6 +116,15 @@ unsigned grid_for(idx_t per_block, idx_t total, unsigned cap) {
 
 double2 ldc(const double* p, unsigned i) { return c2(p[2 * i], p[2 * i + 1]); }
 
+// The operation phase of an item for all threads; a chain runs stage by stage.
+template <class Op>
+bool run_stages(const Op&, const DmGeom&, double2*, unsigned) { return false; }
+bool run_stages(const OpChain& op, const DmGeom& g, double2* vb, unsigned nthr) {
+    for (unsigned i = 0; i < op.nst; ++i)
+        for (unsigned t = 0; t < nthr; ++t) op.stage(i, g, vb, t, nthr);
+    return true;
+}
+
 template <class Map, class Op>
 void run_engine(const EmuMem& mem, const Map& map, const DmGeom& g, const Op& op) {
     const unsigned grid = grid_for(1, g.items, kSms * 32u);
@@ -127,6 +136,7 @@ void run_engine(const EmuMem& mem, const Map& map, const DmGeom& g, const Op& op
         for (idx_t w = b; w < g.items; w += grid) {
             for (int phase = 0; phase < kDmPhases; ++phase) {
                 const unsigned nthr = (phase == 1 || phase == 5) ? kDmIssueThreads : kDmBlock;
+                if (phase == 3 && run_stages(o, g, vb.data(), nthr)) continue;
                 for (unsigned t = 0; t < nthr; ++t)
                     dm_engine_item_phase(phase, mem, map, g, o, w, pd.data(), vb.data(), t, nthr);
             }
@@ -364,6 +374,20 @@ int emu_dm_phase(int layout, unsigned log_tile, double* rho, uint64_t len, unsig
     for (unsigned y = 0; y < 8; ++y) fac.phase[y] = y < (1u << k) ? ldc(phase, y) : c2(1.0, 0.0);
     run_phase(layout, log_tile, mem, n, fac);
     return 0;
+}
+
+// One chain of 1-qubit channels on ascending distinct qubits (k <= 6); -2: they do not fit one
+// staged block.
+int emu_dm_chain(int layout, unsigned log_tile, double* rho, uint64_t len, unsigned n, unsigned k,
+                 const unsigned* qubits, const double* sops, uint32_t* reads, uint32_t* writes, uint64_t* oob) {
+    DmGeom g;
+    unsigned vbit[kChainMax];
+    if (!dm_chain_geometry(n, k, qubits, ls_max_for(layout, log_tile), &g, vbit)) return -2;
+    OpChain op;
+    for (unsigned j = 0; j < kChainMax; ++j)
+        for (unsigned e = 0; e < 16; ++e) op.s[j][e] = j < k ? ldc(sops + 32 * j, e) : c2(0.0, 0.0);
+    dm_chain_stages(op, k, vbit);
+    return engine_dispatch(layout, log_tile, rho, len, n, g, op, reads, writes, oob);
 }
 
 // exp_diag on a density matrix: phase table from diag, then the phase pass (as the GPU path).

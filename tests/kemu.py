@@ -100,6 +100,15 @@ def dm_superop1(layout, lt, data, n, target, sop):
                                              _ptr(r), _ptr(w), C.byref(b)))
 
 
+def dm_chain(layout, lt, data, n, qubits, sops):
+    """A chain of 1-qubit channels on ascending distinct qubits through one staged block."""
+    q = _arr(qubits, np.uint32)
+    s = _arr(np.asarray(sops).reshape(-1), np.complex128)
+    f = lib().emu_dm_chain
+    return _run(f, data, lambda o, r, w, b: (LAYOUT[layout], lt, _ptr(o), C.c_uint64(o.size), n, len(q), _ptr(q),
+                                             _ptr(s), _ptr(r), _ptr(w), C.byref(b)))
+
+
 def dm_superop2(layout, lt, data, n, q0, q1, sop):
     s = _arr(np.asarray(sop).reshape(-1), np.complex128)
     f = lib().emu_dm_superop2
