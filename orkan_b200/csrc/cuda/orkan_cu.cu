@@ -181,6 +181,25 @@ int wait_mapped(const MappedOut& m, unsigned ncomp, cudaStream_t st) {
     return *flag == m.seq ? 0 : (int)cudaErrorUnknown;
 }
 
+// A fused run: persistent blocks, as many as fit (looked up once per chunk size, from which the
+// block's threads and shared memory follow).
+template <int K>
+int launch_fused(void* psi, const FusedPlan& plan, cudaStream_t st) {
+    static std::atomic<int> per_sm[kFuseMaxLog + 1];
+    const unsigned nt = fused_threads(plan);
+    const size_t smem = fused_smem_bytes(plan);
+    int per = per_sm[plan.C].load(std::memory_order_relaxed);
+    if (per < 1) {
+        cudaFuncSetAttribute(k_pure_fused<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pure_fused<K>, (int)nt, smem) != cudaSuccess || per < 1)
+            per = 1;
+        per_sm[plan.C].store(per, std::memory_order_relaxed);
+    }
+    const unsigned grid = grid_for(1, plan.nchunks(), (unsigned)(sm_count() * per));
+    k_pure_fused<K><<<grid, nt, smem, st>>>(FusedDevMem{static_cast<double2*>(psi)}, plan);
+    return finish_launch();
+}
+
 struct DevMemC2 {
     const double2* p;
     __device__ __forceinline__ double2 ld(idx_t i) const { return p[i]; }
@@ -269,26 +288,12 @@ int orkan_cu_pure_fused(void* psi, unsigned n, unsigned log_chunk, unsigned ngat
     if (!psi || !gates) return (int)cudaErrorInvalidValue;
     FusedPlan plan;
     if (!fused_plan(n, log_chunk, ngates, gates, &plan)) return (int)cudaErrorInvalidValue;
-    const size_t smem = fused_smem_bytes(plan);
-    static std::atomic<bool> attr{false};
-    if (!attr.load(std::memory_order_relaxed)) {
-        cudaFuncSetAttribute(k_pure_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        attr.store(true, std::memory_order_relaxed);
+    switch (plan.K) {
+        case 4: return launch_fused<4>(psi, plan, as_stream(stream));
+        case 3: return launch_fused<3>(psi, plan, as_stream(stream));
+        case 2: return launch_fused<2>(psi, plan, as_stream(stream));
+        default: return launch_fused<1>(psi, plan, as_stream(stream));
     }
-    // threads per block: 128 (four blocks per SM at 124 registers; measured 15 % faster than
-    // 256 on a 200-gate random circuit at 30 q), or 256 through the tuning knob
-    // ORKAN_FUSE_THREADS, read once
-    static const unsigned nt = [] {
-        const char* e = getenv("ORKAN_FUSE_THREADS");
-        return (e && atoi(e) == 256) ? kFuseThreads : 128u;
-    }();
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pure_fused, (int)nt, smem) != cudaSuccess ||
-        per_sm < 1)
-        per_sm = 1;
-    const unsigned grid = grid_for(1, plan.nchunks(), (unsigned)(sm_count() * per_sm));
-    k_pure_fused<<<grid, nt, smem, as_stream(stream)>>>(DevMem{static_cast<double2*>(psi)}, plan);
-    return finish_launch();
 }
 
 unsigned long long orkan_cu_fused_need(const orkan_fgate_t* g) { return g ? fused_need(*g) : ~0ull; }

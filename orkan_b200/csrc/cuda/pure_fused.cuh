@@ -6,9 +6,13 @@
 // 2^C amplitudes whose indices differ only in C chosen "local" qubits, it is loaded into
 // shared memory once, every gate of the run is applied to it there, and it is stored once.
 // Inside the chunk the run is cut into stages: a stage holds consecutive gates whose mixed
-// qubits fit a group of 4 local qubits; every thread takes the 16 amplitudes of a set that
+// qubits fit a group of K local qubits; every thread takes the 2^K amplitudes of a set that
 // differ only in the group's qubits into registers, applies all of the stage's gates there,
 // and puts them back, so the shared memory is read and written once per stage, not per gate.
+// K = 4 where the state has many chunks: a gate's decoding is then shared by 16 amplitudes and
+// a run has fewer stages.  K = 3 where one block holds the whole state (up to 12 qubits): the
+// block then has twice the threads and each thread half the arithmetic, which is what a run
+// waits for there.
 //
 // * A gate can join a run when the qubits it mixes are local: the target of X, Y, H, Hy, Rx,
 //   Ry, CX, CY and CCX, both qubits of SWAP.  Controls and diagonal gates (Z, S, Sdg, T, Tdg,
@@ -34,43 +38,52 @@ namespace orkan {
 
 constexpr unsigned kFuseMaxGates = 48;   // gates of one fused launch
 constexpr unsigned kFuseMaxLog = 12;     // chunk of at most 2^12 amplitudes (64 KB)
-constexpr unsigned kFuseThreads = 256;
-constexpr unsigned kFuseVec = 8;         // loads a thread issues before it stores any
-constexpr unsigned kFuseGroup = 3;       // local qubits of a register stage (8 amplitudes)
+constexpr unsigned kFuseThreads = 512;   // threads of a block at most
+constexpr unsigned kFuseGroup = 4;       // local qubits of a register stage at most (16 amplitudes)
 
-enum FKind : unsigned char {
-    kFMix = 0,    // pair_op<op> on (bit t clear, bit t set) where the local controls are set
-    kFPhase,      // the |1>-half of a diagonal 1-qubit op on local bit t (local controls)
-    kFRz,         // Rz on local bit t (both halves change)
-    kFSwap,       // exchange of the (t=1, a=0) and (t=0, a=1) amplitudes
-    kFScale       // diagonal op on non-local bits: every amplitude of the chunk changes
+// What a gate does to a thread's registers v[j], j = the set's element.  A gate acts where the
+// chunk has all bits of gmask, the set all bits of lm and the element all bits of jm.
+enum FOp : unsigned char {
+    kFMix = 0,          // + 4 op + rt: pair_op<op> on elements j, j | 1 << rt (X, Y, H, Hy, Rx, Ry)
+    kFPhase = 24,       // + 5 k + (0: every element, 1 + b: those with bit b): the |1>-factor of diagonal op k
+    kFCz = 54,          // sign of the elements with all bits of jm
+    kFRz = 55,          // + b: Rz, the element's bit b picks the factor
+    kFRzOut = 59,       // Rz, the set's bit lm or the chunk's bit gq - 1 picks the factor
+    kFSwap = 60         // + 0..5: exchange of element bits (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
 };
 
 struct FGate {
-    unsigned char kind, op, t, a;
-    unsigned char rt, ra;      // kFMix / kFSwap: positions of t and a in the stage's group
-    unsigned char pad_[2];
-    unsigned lmask;            // local control bits (chunk index)
-    unsigned long long gmask;  // the gate acts on a chunk only when all these global bits are set
-    unsigned long long gbit;   // kFScale Rz: the global bit that picks the |0> or |1> factor
+    unsigned char h;           // FOp
+    unsigned char jm;
+    unsigned char gq;          // kFRzOut
+    unsigned char pad_;
+    unsigned lm;               // chunk-index bits outside the stage's group
+    unsigned long long gmask;  // global bits
     double c, s;
 };
 
+struct FStage {
+    unsigned char first;                   // first gate
+    unsigned char g[kFuseGroup];           // local bits of the group, ascending
+    unsigned char f[kFuseMaxLog];          // the other local bits: bit i of a set's number goes to bit f[i]
+};
+
 struct FusedPlan {
-    unsigned n, C, m;          // qubits, log2 chunk, length of the run of local bits 0..m-1
+    unsigned n, C;             // qubits, log2 chunk
     unsigned ngates;
+    unsigned nnl;              // non-local bits
     unsigned long long nlmask; // global bits that are not local (the chunk id's bits)
     unsigned char lq[kFuseMaxLog];   // global position of local bit i (ascending)
-    unsigned K;                // qubits of a stage's group: min(kFuseGroup, C)
+    unsigned char nlq[32];     // global position of chunk id bit i (the first 32)
+    unsigned K;                // qubits of a stage's group
     unsigned nstages;
-    unsigned char st_first[kFuseMaxGates + 1];     // first gate of stage s; st_first[nstages] = ngates
-    unsigned char st_g[kFuseMaxGates][kFuseGroup]; // local bits of stage s's group, ascending
+    FStage st[kFuseMaxGates + 1];    // st[nstages].first = ngates
     FGate g[kFuseMaxGates];
     ORKAN_HD unsigned chunk() const { return 1u << C; }
     ORKAN_HD idx_t nchunks() const { return idx_t(1) << (n - C); }
-    ORKAN_HD unsigned ntab() const { return 1u << (C - m); }
     ORKAN_HD unsigned sets() const { return 1u << (C - K); }
 };
+static_assert(sizeof(FusedPlan) <= 4000, "a kernel parameter");
 
 // Global qubits a gate mixes (must be local) as a bit mask; ~0 for an unknown op.
 inline unsigned long long fused_need(const orkan_fgate_t& q) {
@@ -117,94 +130,108 @@ inline bool fused_plan(unsigned n, unsigned C, unsigned ngates, const orkan_fgat
     unsigned i = 0;
     for (unsigned b = 0; b < n; ++b)
         if ((need >> b) & 1ull) { P->lq[i] = (unsigned char)b; pos[b] = i++; }
-    P->m = 0;
-    while (P->m < C && P->lq[P->m] == P->m) ++P->m;
-    for (unsigned gi = 0; gi < ngates; ++gi) {
-        const orkan_fgate_t& q = gates[gi];
-        FGate& f = P->g[gi];
-        f.kind = kFMix;
-        f.op = 0;
-        f.t = f.a = 0;
-        f.lmask = 0;
-        f.gmask = f.gbit = 0;
-        f.c = q.c;
-        f.s = q.s;
-        auto local = [&](unsigned b) { return ((need >> b) & 1ull) != 0; };
-        auto control = [&](unsigned b) {
-            if (local(b)) f.lmask |= 1u << pos[b];
-            else f.gmask |= 1ull << b;
-        };
-        switch (q.op) {
-            case ORKAN_OP_X: case ORKAN_OP_Y: case ORKAN_OP_H: case ORKAN_OP_HY: case ORKAN_OP_RX: case ORKAN_OP_RY:
-                f.kind = kFMix; f.op = (unsigned char)q.op; f.t = (unsigned char)pos[q.q[0]];
-                break;
-            case ORKAN_OP_Z: case ORKAN_OP_S: case ORKAN_OP_SDG: case ORKAN_OP_T: case ORKAN_OP_TDG: case ORKAN_OP_P:
-                f.op = (unsigned char)q.op;
-                if (local(q.q[0])) { f.kind = kFPhase; f.t = (unsigned char)pos[q.q[0]]; }
-                else { f.kind = kFScale; f.gmask = 1ull << q.q[0]; }
-                break;
-            case ORKAN_OP_RZ:
-                f.op = (unsigned char)q.op;
-                if (local(q.q[0])) { f.kind = kFRz; f.t = (unsigned char)pos[q.q[0]]; }
-                else { f.kind = kFScale; f.gbit = 1ull << q.q[0]; }
-                break;
-            case ORKAN_FOP_CX: case ORKAN_FOP_CY:
-                f.kind = kFMix; f.op = q.op == ORKAN_FOP_CX ? (unsigned char)kOpX : (unsigned char)kOpY;
-                f.t = (unsigned char)pos[q.q[1]];
-                control(q.q[0]);
-                break;
-            case ORKAN_FOP_CZ:
-                f.op = (unsigned char)kOpZ;
-                if (local(q.q[1])) { f.kind = kFPhase; f.t = (unsigned char)pos[q.q[1]]; control(q.q[0]); }
-                else if (local(q.q[0])) { f.kind = kFPhase; f.t = (unsigned char)pos[q.q[0]]; control(q.q[1]); }
-                else { f.kind = kFScale; f.gmask = (1ull << q.q[0]) | (1ull << q.q[1]); }
-                break;
-            case ORKAN_FOP_SWAP:
-                f.kind = kFSwap; f.t = (unsigned char)pos[q.q[0]]; f.a = (unsigned char)pos[q.q[1]];
-                break;
-            case ORKAN_FOP_CCX:
-                f.kind = kFMix; f.op = (unsigned char)kOpX; f.t = (unsigned char)pos[q.q[2]];
-                control(q.q[0]);
-                control(q.q[1]);
-                break;
-            default: return false;
-        }
-    }
-    // stages: consecutive gates whose mixed local bits fit a group of K bits; a group with
-    // fewer is filled with the lowest other local bits
-    P->K = C < kFuseGroup ? C : kFuseGroup;
+    P->nnl = n - C;
+    for (unsigned b = 0, k = 0; b < n && k < 32; ++b)
+        if ((P->nlmask >> b) & 1ull) P->nlq[k++] = (unsigned char)b;
+    const unsigned most = C == n ? 3u : kFuseGroup;
+    P->K = C < most ? C : most;
+    // stages: consecutive gates whose mixed local bits fit a group of K bits; a group with fewer is
+    // filled with the lowest other local bits
     P->nstages = 0;
     unsigned cur = 0;
     auto close = [&](unsigned first, unsigned last) {
         for (unsigned b = 0; b < C && popc64(cur) < P->K; ++b) cur |= 1u << b;
-        unsigned char* gb = P->st_g[P->nstages];
-        unsigned k = 0;
+        FStage& st = P->st[P->nstages++];
+        st.first = (unsigned char)first;
+        unsigned k = 0, e[kFuseMaxLog] = {};             // element bit of a local bit of the group
         for (unsigned b = 0; b < C; ++b)
-            if ((cur >> b) & 1u) gb[k++] = (unsigned char)b;
-        for (; k < kFuseGroup; ++k) gb[k] = 0;
+            if ((cur >> b) & 1u) { e[b] = k; st.g[k++] = (unsigned char)b; }
+        for (; k < kFuseGroup; ++k) st.g[k] = 0;
+        // lanes: the three lowest bits of a set's number go to free bits of different residues mod 3
+        // where there are such, which fused_phys spreads over the shared-memory banks
+        unsigned left = (P->chunk() - 1) & ~cur, nf = 0;
+        for (unsigned r = 0; r < 3; ++r)
+            for (unsigned b = 0; b < C; ++b)
+                if (((left >> b) & 1u) && b % 3 == r) {
+                    st.f[nf++] = (unsigned char)b;
+                    left &= ~(1u << b);
+                    break;
+                }
+        for (unsigned b = 0; b < C; ++b)
+            if ((left >> b) & 1u) st.f[nf++] = (unsigned char)b;
+        for (; nf < kFuseMaxLog; ++nf) st.f[nf] = 0;
         for (unsigned gi = first; gi < last; ++gi) {
-            FGate& f = P->g[gi];
-            f.rt = f.ra = 0;
-            for (unsigned r = 0; r < P->K; ++r) {
-                if (gb[r] == f.t) f.rt = (unsigned char)r;
-                if (gb[r] == f.a) f.ra = (unsigned char)r;
+            const orkan_fgate_t& q = gates[gi];
+            FGate f{};
+            f.c = q.c;
+            f.s = q.s;
+            auto local = [&](unsigned b) { return ((need >> b) & 1ull) != 0; };
+            auto grouped = [&](unsigned b) { return local(b) && ((cur >> pos[b]) & 1u); };
+            auto bit = [&](unsigned b) { return e[pos[b]]; };
+            auto control = [&](unsigned b) {
+                if (grouped(b)) f.jm |= (unsigned char)(1u << bit(b));
+                else if (local(b)) f.lm |= 1u << pos[b];
+                else f.gmask |= 1ull << b;
+            };
+            switch (q.op) {
+                case ORKAN_OP_X: case ORKAN_OP_Y: case ORKAN_OP_H: case ORKAN_OP_HY: case ORKAN_OP_RX: case ORKAN_OP_RY: {
+                    const unsigned k6 = q.op == ORKAN_OP_X ? 0 : q.op == ORKAN_OP_Y ? 1 : q.op == ORKAN_OP_H ? 2
+                                        : q.op == ORKAN_OP_HY ? 3 : q.op == ORKAN_OP_RX ? 4 : 5;
+                    f.h = (unsigned char)(kFMix + 4 * k6 + bit(q.q[0]));
+                    break;
+                }
+                case ORKAN_FOP_CX: case ORKAN_FOP_CY:
+                    f.h = (unsigned char)(kFMix + 4 * (q.op == ORKAN_FOP_CX ? 0 : 1) + bit(q.q[1]));
+                    control(q.q[0]);
+                    break;
+                case ORKAN_FOP_CCX:
+                    f.h = (unsigned char)(kFMix + bit(q.q[2]));
+                    control(q.q[0]);
+                    control(q.q[1]);
+                    break;
+                case ORKAN_OP_Z: case ORKAN_OP_S: case ORKAN_OP_SDG: case ORKAN_OP_T: case ORKAN_OP_TDG: case ORKAN_OP_P: {
+                    const unsigned k6 = q.op == ORKAN_OP_Z ? 0 : q.op == ORKAN_OP_S ? 1 : q.op == ORKAN_OP_SDG ? 2
+                                        : q.op == ORKAN_OP_T ? 3 : q.op == ORKAN_OP_TDG ? 4 : 5;
+                    if (grouped(q.q[0])) f.h = (unsigned char)(kFPhase + 5 * k6 + 1 + bit(q.q[0]));
+                    else { f.h = (unsigned char)(kFPhase + 5 * k6); control(q.q[0]); }
+                    break;
+                }
+                case ORKAN_FOP_CZ:
+                    control(q.q[0]);
+                    control(q.q[1]);
+                    f.h = kFCz;
+                    break;
+                case ORKAN_OP_RZ:
+                    if (grouped(q.q[0])) f.h = (unsigned char)(kFRz + bit(q.q[0]));
+                    else {
+                        f.h = kFRzOut;
+                        if (local(q.q[0])) f.lm = 1u << pos[q.q[0]];
+                        else f.gq = (unsigned char)(q.q[0] + 1);
+                    }
+                    break;
+                default: {                               // SWAP
+                    unsigned x = bit(q.q[0]), y = bit(q.q[1]);
+                    if (x > y) { const unsigned t = x; x = y; y = t; }
+                    f.h = (unsigned char)(kFSwap + (x == 0 ? y - 1 : x == 1 ? y + 1 : 5u));
+                    break;
+                }
             }
+            P->g[gi] = f;
         }
-        P->st_first[P->nstages++] = (unsigned char)first;
         cur = 0;
     };
     unsigned first = 0;
     for (unsigned gi = 0; gi < ngates; ++gi) {
-        const FGate& f = P->g[gi];
-        const unsigned need = f.kind == kFMix ? (1u << f.t) : f.kind == kFSwap ? ((1u << f.t) | (1u << f.a)) : 0u;
-        if (popc64(cur | need) > P->K) {
+        unsigned mixed = 0;
+        for (unsigned long long r = fused_need(gates[gi]); r; r &= r - 1) mixed |= 1u << pos[ctz64(r)];
+        if (popc64(cur | mixed) > P->K) {
             close(first, gi);
             first = gi;
         }
-        cur |= need;
+        cur |= mixed;
     }
     close(first, ngates);
-    P->st_first[P->nstages] = (unsigned char)ngates;
+    P->st[P->nstages].first = (unsigned char)ngates;
     return true;
 }
 
@@ -215,6 +242,15 @@ ORKAN_HD unsigned fused_phys(unsigned s) { return s ^ (((s >> 3) ^ (s >> 6) ^ (s
 
 // Global index of the chunk's amplitude 0: the chunk id's bits deposited on the non-local bits.
 ORKAN_HD idx_t fused_base(const FusedPlan& P, idx_t chunk) {
+#ifdef __CUDA_ARCH__
+    if (P.nnl <= 32) {                               // one bit per lane
+        const unsigned lane = threadIdx.x & 31u;
+        const idx_t one = lane < P.nnl && ((chunk >> lane) & 1u) ? idx_t(1) << P.nlq[lane] : 0;
+        const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)one);
+        const unsigned hi = P.n <= 32 ? 0u : __reduce_or_sync(0xffffffffu, (unsigned)(one >> 32));
+        return ((idx_t)hi << 32) | lo;
+    }
+#endif
     idx_t base = 0;
     unsigned long long rest = P.nlmask;
     while (rest && chunk) {
@@ -226,256 +262,267 @@ ORKAN_HD idx_t fused_base(const FusedPlan& P, idx_t chunk) {
     return base;
 }
 
-// Offset table of the local bits above the contiguous run: tab[h] = sum of bit i of h at
-// global position lq[m + i].
-ORKAN_HD void fused_table(const FusedPlan& P, idx_t* tab, unsigned tid, unsigned nthr) {
-    for (unsigned h = tid; h < P.ntab(); h += nthr) {
-        idx_t o = 0;
-        for (unsigned i = 0; i + P.m < P.C; ++i) o |= idx_t((h >> i) & 1u) << P.lq[P.m + i];
-        tab[h] = o;
+// Global offset of chunk index j: its bits at the local bits' global positions.
+ORKAN_HD idx_t fused_off(const FusedPlan& P, unsigned j) {
+    idx_t o = 0;
+#pragma unroll
+    for (unsigned i = 0; i < kFuseMaxLog; ++i)
+        if (i < P.C) o |= idx_t((j >> i) & 1u) << P.lq[i];
+    return o;
+}
+
+// A thread's share of a chunk for load and store: the 2^K amplitudes j = tid | u << (C - K), whose
+// offsets and slots are those of tid with the bits of u added, so that an amplitude costs a few
+// logic instructions.  Mem::cp16(dst, x) copies amplitude x (asynchronously on the GPU).
+struct FusedWalk {
+    idx_t off;                 // fused_off(tid)
+    unsigned slot;             // fused_phys(tid)
+    bool live;                 // tid names a share
+};
+ORKAN_HD FusedWalk fused_walk(const FusedPlan& P, unsigned tid) {
+    FusedWalk w;
+    w.live = tid < P.sets();
+    w.off = fused_off(P, tid);
+    w.slot = fused_phys(tid);
+    return w;
+}
+template <int K, class F>
+ORKAN_HD void fused_each(const FusedPlan& P, const FusedWalk& w, const F& f) {
+    if (!w.live) return;
+    idx_t go[K];
+    unsigned so[K];
+#pragma unroll
+    for (int b = 0; b < K; ++b) {
+        go[b] = idx_t(1) << P.lq[P.C - K + b];
+        so[b] = fused_phys(1u << (P.C - K + b));
+    }
+#pragma unroll
+    for (int u = 0; u < (1 << K); ++u) {
+        idx_t o = w.off;
+        unsigned s = w.slot;
+#pragma unroll
+        for (int b = 0; b < K; ++b)
+            if ((u >> b) & 1) {
+                o |= go[b];
+                s ^= so[b];
+            }
+        f(o, s);
     }
 }
-
-ORKAN_HD idx_t fused_off(const FusedPlan& P, const idx_t* tab, unsigned j) {
-    return tab[j >> P.m] + (j & ((1u << P.m) - 1u));
+template <int K, class Mem>
+ORKAN_HD void fused_load(const Mem& mem, const FusedPlan& P, const FusedWalk& w, idx_t base, double2* buf) {
+    fused_each<K>(P, w, [&](idx_t o, unsigned s) { mem.cp16(buf + s, base | o); });
 }
-
-template <class Mem>
-ORKAN_HD void fused_load(const Mem& mem, const FusedPlan& P, const idx_t* tab, idx_t base, double2* buf,
-                         unsigned tid, unsigned nthr) {
-    const unsigned N = P.chunk();
-    for (unsigned j0 = tid; j0 < N; j0 += kFuseVec * nthr) {
-        double2 v[kFuseVec];
-#pragma unroll
-        for (unsigned u = 0; u < kFuseVec; ++u) {
-            const unsigned j = j0 + u * nthr;
-            if (j < N) v[u] = mem.ld(base + fused_off(P, tab, j));
-        }
-#pragma unroll
-        for (unsigned u = 0; u < kFuseVec; ++u) {
-            const unsigned j = j0 + u * nthr;
-            if (j < N) buf[fused_phys(j)] = v[u];
-        }
-    }
+template <int K, class Mem>
+ORKAN_HD void fused_store(const Mem& mem, const FusedPlan& P, const FusedWalk& w, idx_t base, const double2* buf) {
+    fused_each<K>(P, w, [&](idx_t o, unsigned s) { mem.st(base | o, buf[s]); });
 }
-
-template <class Mem>
-ORKAN_HD void fused_store(const Mem& mem, const FusedPlan& P, const idx_t* tab, idx_t base, const double2* buf,
-                          unsigned tid, unsigned nthr) {
-    const unsigned N = P.chunk();
-    for (unsigned j = tid; j < N; j += nthr) mem.st(base + fused_off(P, tab, j), buf[fused_phys(j)]);
-}
-
-// Does gate g act on the chunk at base?  (Its non-local controls are all set.)
-ORKAN_HD bool fused_active(const FGate& g, idx_t base) { return (base & g.gmask) == g.gmask; }
 
 // ---- register stages -------------------------------------------------------------------
-// v[j] holds the amplitude at chunk index idx[j] = set base | (bit b of j at group bit g[b]).
+// v[j] holds the amplitude at chunk index sb | (bit b of j at group bit g[b]).
 
+//
+// Where a gate has a condition, the new value is computed and selected instead of branched to, and
+// exchanges are selects on the condition even where there is none (`on` is then true, which the
+// compiler cannot know).  A divergent branch, or an exchange that the compiler may carry out by
+// renaming registers, makes it copy all 64 registers of the 16 amplitudes at the switch's ends:
+// 284 instructions per H and 342 per X then, 92 and 150 now (64 and 0 of them arithmetic).
+ORKAN_HD double2 reg_select(bool p, double2 a, double2 b) { return c2(p ? a.x : b.x, p ? a.y : b.y); }
+
+// X and Y on element bit RT where the set (on) and the element have the controls.
 template <int OP, int RT, int NV>
-ORKAN_HD void reg_mix(double2 (&v)[NV], const unsigned (&idx)[NV], const FGate& g) {
-    const double c = g.c, s = g.s;
-    if (g.lmask == 0) {                              // no local control: every pair
+ORKAN_HD void reg_flip(double2 (&v)[NV], const FGate& g, bool on) {
+    if constexpr ((1 << RT) < NV) {
 #pragma unroll
         for (int j = 0; j < NV; ++j)
-            if (!(j & (1 << RT))) pair_op<OP>(v[j], v[j | (1 << RT)], c, s);
-        return;
-    }
-#pragma unroll
-    for (int j = 0; j < NV; ++j)
-        if (!(j & (1 << RT)) && (idx[j] & g.lmask) == g.lmask) pair_op<OP>(v[j], v[j | (1 << RT)], c, s);
-}
-
-template <int OP, int NV>
-ORKAN_HD void reg_mix_at(double2 (&v)[NV], const unsigned (&idx)[NV], const FGate& g) {
-    switch (g.rt) {
-        case 0: reg_mix<OP, 0>(v, idx, g); break;
-        case 1: if (NV > 2) reg_mix<OP, (NV > 2 ? 1 : 0)>(v, idx, g); break;
-        case 2: if (NV > 4) reg_mix<OP, (NV > 4 ? 2 : 0)>(v, idx, g); break;
-        default: if (NV > 8) reg_mix<OP, (NV > 8 ? 3 : 0)>(v, idx, g); break;
+            if (!(j & (1 << RT))) {
+                const bool p = on && (j & g.jm) == g.jm;
+                const double2 a = v[j], b = v[j | (1 << RT)];
+                double2 na = a, nb = b;
+                pair_op<OP>(na, nb, 0.0, 0.0);
+                v[j] = reg_select(p, na, a);
+                v[j | (1 << RT)] = reg_select(p, nb, b);
+            }
     }
 }
 
-// The |1>-half op of a diagonal gate on local bit t (its bit need not be in the group).
-template <int OP, int NV>
-ORKAN_HD void reg_phase(double2 (&v)[NV], const unsigned (&idx)[NV], const FGate& g) {
-    const unsigned need = g.lmask | (1u << g.t);
+// H, Hy, Rx, Ry on element bit RT (they have no controls).
+template <int OP, int RT, int NV>
+ORKAN_HD void reg_mix(double2 (&v)[NV], const FGate& g) {
+    if constexpr ((1 << RT) < NV) {
 #pragma unroll
-    for (int j = 0; j < NV; ++j)
-        if ((idx[j] & need) == need) {
-            double2 a = c2(0.0, 0.0);
-            pair_op<OP>(a, v[j], g.c, g.s);
-        }
+        for (int j = 0; j < NV; ++j)
+            if (!(j & (1 << RT))) pair_op<OP>(v[j], v[j | (1 << RT)], g.c, g.s);
+    }
 }
 
-// Rz on local bit t: each amplitude takes the |0> or the |1> factor by its bit t (or, on a
-// non-local bit, by the chunk's bit: `one`).
-// The |1> factor is the |0> factor with s negated: (c x + s y, c y - s x) -> (c x - s y, c y + s x),
-// the same roundings as pair_op<kOpRz>.
+// A diagonal 1-qubit op's |1>-factor on the elements with bit B (no condition then), or, B < 0, on all
+// elements of the sets that have the bit (on).
+template <int OP, int B, int NV>
+ORKAN_HD void reg_phase(double2 (&v)[NV], const FGate& g, bool on) {
+    if constexpr (B < 0 || (1 << (B < 0 ? 0 : B)) < NV) {
+        constexpr bool plain = B >= 0 && OP != kOpS && OP != kOpSdg;     // S exchanges re and im
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+            if (B < 0 || ((j >> (B < 0 ? 0 : B)) & 1)) {
+                double2 a = c2(0.0, 0.0), x = v[j];
+                pair_op<OP>(a, x, g.c, g.s);
+                v[j] = plain ? x : reg_select(on, x, v[j]);
+            }
+    }
+}
+
 template <int NV>
-ORKAN_HD void reg_rz(double2 (&v)[NV], const unsigned (&idx)[NV], const FGate& g, bool local, bool one) {
+ORKAN_HD void reg_cz(double2 (&v)[NV], const FGate& g, bool on) {
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-        const double s = (local ? ((idx[j] >> g.t) & 1u) != 0 : one) ? -g.s : g.s;
-        v[j] = c2(lin2(g.c, v[j].x, s, v[j].y), lin2(g.c, v[j].y, -s, v[j].x));
+        double2 a = c2(0.0, 0.0), x = v[j];
+        pair_op<kOpZ>(a, x, 0.0, 0.0);
+        v[j] = reg_select(on && (j & g.jm) == g.jm, x, v[j]);
     }
 }
 
-// A diagonal 1-qubit op's |1> factor on every amplitude (a non-local gate whose bits are set).
-template <int OP, int NV>
-ORKAN_HD void reg_scale(double2 (&v)[NV], const FGate& g) {
+// Rz: the |1> factor is the |0> factor with s negated, (c x + s y, c y - s x) -> (c x - s y, c y + s x),
+// the same roundings as pair_op<kOpRz>.  B < 0: every element takes the factor that `one` picks.
+template <int B, int NV>
+ORKAN_HD void reg_rz(double2 (&v)[NV], const FGate& g, bool one) {
+    if constexpr (B < 0 || (1 << (B < 0 ? 0 : B)) < NV) {
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        double2 a = c2(0.0, 0.0);
-        pair_op<OP>(a, v[j], g.c, g.s);
-    }
-}
-
-template <int RT, int RA, int NV>
-ORKAN_HD void reg_swap(double2 (&v)[NV]) {
-#pragma unroll
-    for (int j = 0; j < NV; ++j)
-        if (!(j & (1 << RT)) && !(j & (1 << RA))) {
-            const double2 x = v[j | (1 << RT)];
-            v[j | (1 << RT)] = v[j | (1 << RA)];
-            v[j | (1 << RA)] = x;
+        for (int j = 0; j < NV; ++j) {
+            const double s = (B < 0 ? one : (bool)((j >> (B < 0 ? 0 : B)) & 1)) ? -g.s : g.s;
+            v[j] = c2(lin2(g.c, v[j].x, s, v[j].y), lin2(g.c, v[j].y, -s, v[j].x));
         }
-}
-
-template <int NV>
-ORKAN_HD void reg_swap_at(double2 (&v)[NV], unsigned rt, unsigned ra) {
-    constexpr int K = NV >= 16 ? 4 : NV >= 8 ? 3 : NV >= 4 ? 2 : 1;
-    const unsigned lo = rt < ra ? rt : ra, hi = rt < ra ? ra : rt;
-    if (K < 2) return;
-    switch (lo * 4 + hi) {
-        case 1: reg_swap<0, 1>(v); break;
-        case 2: if (K > 2) reg_swap<0, (K > 2 ? 2 : 1)>(v); break;
-        case 3: if (K > 3) reg_swap<0, (K > 3 ? 3 : 1)>(v); break;
-        case 6: if (K > 2) reg_swap<1, (K > 2 ? 2 : 0)>(v); break;
-        case 7: if (K > 3) reg_swap<1, (K > 3 ? 3 : 0)>(v); break;
-        default: if (K > 3) reg_swap<2, (K > 3 ? 3 : 0)>(v); break;   // (2, 3)
     }
 }
 
-// One gate of a stage on a thread's registers.
+template <int X, int Y, int NV>
+ORKAN_HD void reg_swap(double2 (&v)[NV], bool on) {
+    if constexpr ((1 << Y) < NV) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+            if (!(j & (1 << X)) && !(j & (1 << Y))) {
+                const double2 a = v[j | (1 << X)], b = v[j | (1 << Y)];
+                v[j | (1 << X)] = reg_select(on, b, a);
+                v[j | (1 << Y)] = reg_select(on, a, b);
+            }
+    }
+}
+
+// One gate of a stage on a thread's registers: one jump per gate, everything a case needs known
+// at compile time but the angles and conditions.
 template <int NV>
-ORKAN_HD void fused_apply(const FGate& g, double2 (&v)[NV], const unsigned (&idx)[NV], idx_t base) {
-    switch (g.kind) {
-        case kFMix:
-            switch (g.op) {
-                case kOpX: reg_mix_at<kOpX>(v, idx, g); break;
-                case kOpY: reg_mix_at<kOpY>(v, idx, g); break;
-                case kOpH: reg_mix_at<kOpH>(v, idx, g); break;
-                case kOpHy: reg_mix_at<kOpHy>(v, idx, g); break;
-                case kOpRx: reg_mix_at<kOpRx>(v, idx, g); break;
-                default: reg_mix_at<kOpRy>(v, idx, g); break;
-            }
-            break;
-        case kFPhase:
-            switch (g.op) {
-                case kOpZ: reg_phase<kOpZ>(v, idx, g); break;
-                case kOpS: reg_phase<kOpS>(v, idx, g); break;
-                case kOpSdg: reg_phase<kOpSdg>(v, idx, g); break;
-                case kOpT: reg_phase<kOpT>(v, idx, g); break;
-                case kOpTdg: reg_phase<kOpTdg>(v, idx, g); break;
-                default: reg_phase<kOpP>(v, idx, g); break;
-            }
-            break;
-        case kFRz:
-            reg_rz(v, idx, g, true, false);
-            break;
-        case kFSwap:
-            reg_swap_at(v, g.rt, g.ra);
-            break;
-        default:   // kFScale
-            if (g.op == kOpRz) {
-                reg_rz(v, idx, g, false, (base & g.gbit) != 0);
-            } else {
-                switch (g.op) {
-                    case kOpZ: reg_scale<kOpZ>(v, g); break;
-                    case kOpS: reg_scale<kOpS>(v, g); break;
-                    case kOpSdg: reg_scale<kOpSdg>(v, g); break;
-                    case kOpT: reg_scale<kOpT>(v, g); break;
-                    case kOpTdg: reg_scale<kOpTdg>(v, g); break;
-                    default: reg_scale<kOpP>(v, g); break;
-                }
-            }
-            break;
+ORKAN_HD void fused_apply(const FGate& g, double2 (&v)[NV], unsigned sb, idx_t base) {
+    if ((base & g.gmask) != g.gmask) return;                 // the same for the whole block
+    const bool on = g.h == kFRzOut || (sb & g.lm) == g.lm;
+    switch (g.h) {
+#define ORKAN_RT(F, K6, OP, A) \
+    case kFMix + 4 * K6: F<OP, 0> A; break; \
+    case kFMix + 4 * K6 + 1: F<OP, 1> A; break; \
+    case kFMix + 4 * K6 + 2: F<OP, 2> A; break; \
+    case kFMix + 4 * K6 + 3: F<OP, 3> A; break;
+        ORKAN_RT(reg_flip, 0, kOpX, (v, g, on)) ORKAN_RT(reg_flip, 1, kOpY, (v, g, on))
+        ORKAN_RT(reg_mix, 2, kOpH, (v, g)) ORKAN_RT(reg_mix, 3, kOpHy, (v, g))
+        ORKAN_RT(reg_mix, 4, kOpRx, (v, g)) ORKAN_RT(reg_mix, 5, kOpRy, (v, g))
+#undef ORKAN_RT
+#define ORKAN_PH1(K6, OP, B) case kFPhase + 5 * K6 + 1 + (B): reg_phase<OP, B>(v, g, on); break;
+#define ORKAN_PH(K6, OP) ORKAN_PH1(K6, OP, -1) ORKAN_PH1(K6, OP, 0) ORKAN_PH1(K6, OP, 1) ORKAN_PH1(K6, OP, 2) \
+    ORKAN_PH1(K6, OP, 3)
+        ORKAN_PH(0, kOpZ) ORKAN_PH(1, kOpS) ORKAN_PH(2, kOpSdg) ORKAN_PH(3, kOpT) ORKAN_PH(4, kOpTdg) ORKAN_PH(5, kOpP)
+#undef ORKAN_PH
+#undef ORKAN_PH1
+        case kFCz: reg_cz(v, g, on); break;
+        case kFRz: reg_rz<0>(v, g, false); break;
+        case kFRz + 1: reg_rz<1>(v, g, false); break;
+        case kFRz + 2: reg_rz<2>(v, g, false); break;
+        case kFRz + 3: reg_rz<3>(v, g, false); break;
+        case kFRzOut: reg_rz<-1>(v, g, (sb & g.lm) != 0 || (g.gq && ((base >> (g.gq - 1)) & 1u))); break;
+        case kFSwap: reg_swap<0, 1>(v, on); break;
+        case kFSwap + 1: reg_swap<0, 2>(v, on); break;
+        case kFSwap + 2: reg_swap<0, 3>(v, on); break;
+        case kFSwap + 3: reg_swap<1, 2>(v, on); break;
+        case kFSwap + 4: reg_swap<1, 3>(v, on); break;
+        case kFSwap + 5: reg_swap<2, 3>(v, on); break;
+        default: break;
     }
 }
 
 // Stage s of the run on the staged chunk (all threads of the block; a barrier follows).
-// Thread tid takes sets tid, tid + nthr, ...: the set's 2^K amplitudes go to registers, every
-// gate of the stage whose chunk condition holds is applied, and they go back.
-template <int NV>
-ORKAN_HD void fused_stage_k(const FusedPlan& P, unsigned s, idx_t base, double2* buf, unsigned tid, unsigned nthr) {
-    constexpr int K = NV >= 16 ? 4 : NV >= 8 ? 3 : NV >= 4 ? 2 : 1;
-    // element j of a set sits at set base | off[j]; the swizzle is linear over disjoint bits,
-    // so its slot is phys(set base) ^ phys(off[j]), with phys(off[j]) formed once per stage
-    unsigned off[NV], poff[NV];
+// Thread tid takes set tid: the set's 2^K amplitudes go to registers, every gate of the stage
+// whose chunk condition holds is applied, and they go back.  The swizzle is
+// linear over disjoint bits, so element j lies at phys(sb) ^ phys(its group bits).
+template <int K>
+ORKAN_HD void fused_stage_k(const FusedPlan& P, unsigned s, idx_t base, double2* buf, unsigned r) {
+    constexpr int NV = 1 << K;
+    const FStage& st = P.st[s];
+    const unsigned g0 = st.first, g1 = P.st[s + 1].first, nf = P.C - K;
+    unsigned ph[K];
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        unsigned o = 0;
+    for (int b = 0; b < K; ++b) ph[b] = fused_phys(1u << st.g[b]) * 16u;
+    if (r >= P.sets()) return;
+    unsigned sb = 0;
+#pragma unroll
+    for (unsigned i = 0; i < kFuseMaxLog - K; ++i)
+        if (i < nf) sb |= ((r >> i) & 1u) << st.f[i];
+    const unsigned psb = fused_phys(sb) * 16u;
+    unsigned char* raw = reinterpret_cast<unsigned char*>(buf);
+    auto at = [&](int j) -> double2& {
+        unsigned a = psb;
 #pragma unroll
         for (int b = 0; b < K; ++b)
-            if ((j >> b) & 1) o |= 1u << P.st_g[s][b];
-        off[j] = o;
-        poff[j] = fused_phys(o);
-    }
-    const unsigned g0 = P.st_first[s], g1 = P.st_first[s + 1];
-    for (unsigned r = tid; r < P.sets(); r += nthr) {
-        unsigned sb = r;
-        for (int b = 0; b < K; ++b) sb = (unsigned)insert0(sb, P.st_g[s][b]);   // ascending positions
-        const unsigned psb = fused_phys(sb);
-        double2 v[NV];
-        unsigned idx[NV];
+            if ((j >> b) & 1) a ^= ph[b];
+        return *reinterpret_cast<double2*>(raw + a);
+    };
+    double2 v[NV];
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            idx[j] = sb | off[j];
-            v[j] = buf[psb ^ poff[j]];
-        }
-        for (unsigned gi = g0; gi < g1; ++gi) {
-            const FGate& g = P.g[gi];
-            if (fused_active(g, base)) fused_apply(g, v, idx, base);
-        }
+    for (int j = 0; j < NV; ++j) v[j] = at(j);
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+    for (unsigned gi = g0; gi < g1; ++gi) fused_apply(P.g[gi], v, sb, base);
 #pragma unroll
-        for (int j = 0; j < NV; ++j) buf[psb ^ poff[j]] = v[j];
-    }
+    for (int j = 0; j < NV; ++j) at(j) = v[j];
 }
 
-ORKAN_HD void fused_stage(const FusedPlan& P, unsigned s, idx_t base, double2* buf, unsigned tid, unsigned nthr) {
-    switch (P.K) {
-        case 4: fused_stage_k<(kFuseGroup >= 4 ? 16 : 8)>(P, s, base, buf, tid, nthr); break;
-        case 3: fused_stage_k<8>(P, s, base, buf, tid, nthr); break;
-        case 2: fused_stage_k<4>(P, s, base, buf, tid, nthr); break;
-        default: fused_stage_k<2>(P, s, base, buf, tid, nthr); break;
-    }
-}
+// Shared memory of one block: the chunk.
+ORKAN_HD size_t fused_smem_bytes(const FusedPlan& P) { return (size_t)P.chunk() * sizeof(double2); }
 
-// Shared memory of one block: the chunk and the offset table.
-ORKAN_HD size_t fused_smem_bytes(const FusedPlan& P) {
-    return (size_t)P.chunk() * sizeof(double2) + (size_t)P.ntab() * sizeof(idx_t);
-}
+// Threads of a block: one set each, whole warps (at most kFuseThreads: 2^12 amplitudes, K >= 3).
+inline unsigned fused_threads(const FusedPlan& P) { return P.sets() < 32 ? 32u : P.sets(); }
 
 #ifdef __CUDACC__
+struct FusedDevMem {
+    double2* p;
+    __device__ __forceinline__ void st(idx_t i, double2 v) const { p[i] = v; }
+    __device__ __forceinline__ void cp16(double2* dst, idx_t i) const {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                     "l"(p + i) : "memory");
+    }
+};
+
 // Persistent blocks walk the chunks; every gate whose chunk condition holds is applied in
 // shared memory between one load and one store of the chunk.
-__global__ void __launch_bounds__(kFuseThreads) k_pure_fused(DevMem mem, const __grid_constant__ FusedPlan P) {
-    extern __shared__ __align__(16) double2 fbuf[];
-    idx_t* tab = reinterpret_cast<idx_t*>(fbuf + P.chunk());
-    const unsigned tid = threadIdx.x, nthr = blockDim.x;
-    fused_table(P, tab, tid, nthr);
-    __syncthreads();
+//
+// Bound: instruction issue.  A chunk's load, store and one stage take 26 instructions per amplitude, a
+// gate 3 to 10 (the arithmetic of an H is 4), a further stage 5; HBM takes 5.3 ms of the 9.3 ms that a run
+// of 15 random gates takes at 30 qubits (15.1 ms with 8-amplitude sets whose gates copied registers).
+// 200 random gates: 30 qubits 124.7 ms (208.7 before), 12 qubits, one block, 117 us on the GPU (277).
+template <int K>
+__global__ void __launch_bounds__(K == 4 ? 256 : kFuseThreads, K == 4 ? 2 : 1)
+    k_pure_fused(FusedDevMem mem, const __grid_constant__ FusedPlan P) {
+    extern __shared__ __align__(128) double2 fbuf[];
+    const unsigned tid = threadIdx.x;
+    const FusedWalk w = fused_walk(P, tid);
     const idx_t nch = P.nchunks();
     for (idx_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
         const idx_t base = fused_base(P, ch);
-        fused_load(mem, P, tab, base, fbuf, tid, nthr);
+        fused_load<K>(mem, P, w, base, fbuf);
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
         for (unsigned st = 0; st < P.nstages; ++st) {
-            fused_stage(P, st, base, fbuf, tid, nthr);
+            fused_stage_k<K>(P, st, base, fbuf, tid);
             __syncthreads();
         }
-        fused_store(mem, P, tab, base, fbuf, tid, nthr);
+        fused_store<K>(mem, P, w, base, fbuf);
         __syncthreads();
     }
 }

@@ -478,27 +478,40 @@ int emu_fill(double* data, uint64_t len, double re, double im, unsigned corner_l
     return 0;
 }
 
-// A fused run of statevector gates (k_pure_fused): every block of the grid, phase by phase
-// (offset table; per chunk: load, each register stage, store), with a block-local chunk buffer.
+// A fused run of statevector gates (k_pure_fused): every block of the grid, phase by phase (per
+// chunk: load, each register stage, store), with a block-local chunk buffer.
+}  // extern "C"
+
+namespace {
+template <int K>
+void run_fused(const EmuMem& mem, const FusedPlan& P, unsigned grid_cap) {
+    const unsigned nthr = fused_threads(P);
+    const idx_t nch = P.nchunks();
+    const unsigned grid = grid_for(1, nch, grid_cap ? grid_cap : kSms * 4u);
+    std::vector<double2> buf(P.chunk());
+    for (unsigned b = 0; b < grid; ++b)
+        for (idx_t ch = b; ch < nch; ch += grid) {
+            const idx_t base = fused_base(P, ch);
+            for (unsigned t = 0; t < nthr; ++t) fused_load<K>(mem, P, fused_walk(P, t), base, buf.data());
+            for (unsigned st = 0; st < P.nstages; ++st)
+                for (unsigned t = 0; t < nthr; ++t) fused_stage_k<K>(P, st, base, buf.data(), t);
+            for (unsigned t = 0; t < nthr; ++t) fused_store<K>(mem, P, fused_walk(P, t), base, buf.data());
+        }
+}
+}  // namespace
+
+extern "C" {
+
 int emu_pure_fused(double* psi, unsigned n, unsigned log_chunk, unsigned ngates, const orkan_fgate_t* gates,
                    unsigned grid_cap, uint32_t* reads, uint32_t* writes, uint64_t* oob) {
     FusedPlan P;
     if (!fused_plan(n, log_chunk, ngates, gates, &P)) return -1;
-    const unsigned nthr = kFuseThreads;
-    const idx_t nch = P.nchunks();
-    const unsigned grid = grid_for(1, nch, grid_cap ? grid_cap : kSms * 4u);
-    EmuMem mem{reinterpret_cast<double2*>(psi), idx_t(1) << n, reads, writes, oob};
-    std::vector<double2> buf(P.chunk());
-    std::vector<idx_t> tab(P.ntab());
-    for (unsigned b = 0; b < grid; ++b) {
-        for (unsigned t = 0; t < nthr; ++t) fused_table(P, tab.data(), t, nthr);
-        for (idx_t ch = b; ch < nch; ch += grid) {
-            const idx_t base = fused_base(P, ch);
-            for (unsigned t = 0; t < nthr; ++t) fused_load(mem, P, tab.data(), base, buf.data(), t, nthr);
-            for (unsigned st = 0; st < P.nstages; ++st)
-                for (unsigned t = 0; t < nthr; ++t) fused_stage(P, st, base, buf.data(), t, nthr);
-            for (unsigned t = 0; t < nthr; ++t) fused_store(mem, P, tab.data(), base, buf.data(), t, nthr);
-        }
+    const EmuMem mem{reinterpret_cast<double2*>(psi), idx_t(1) << n, reads, writes, oob};
+    switch (P.K) {
+        case 4: run_fused<4>(mem, P, grid_cap); break;
+        case 3: run_fused<3>(mem, P, grid_cap); break;
+        case 2: run_fused<2>(mem, P, grid_cap); break;
+        default: run_fused<1>(mem, P, grid_cap); break;
     }
     return 0;
 }
