@@ -4,6 +4,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "dm_direct.cuh"
 #include "dm_phase.cuh"
 
 namespace orkan {
@@ -32,9 +33,21 @@ inline unsigned grid_for(idx_t work_per_block_units, idx_t total_units, unsigned
 // knob ORKAN_PHASE_ITEMS, read once.
 unsigned phase_items_per_block();
 
-// Elementwise phase pass over a packed (layout 1) or tiled (layout 2) density matrix.
+// Threads one per index of a 2^bits range.
+inline unsigned direct_grid(unsigned bits) { return grid_for(kDirectThreads, idx_t(1) << bits, kFullGrid); }
+
+// Elementwise phase pass over a packed (layout 1) or tiled (layout 2) density matrix: one thread per element
+// up to kDirectSmall qubits (8 q: 4.0 against 6.2 us; from 11 q on the pass that skips whole inactive items
+// is faster, 8.3 against 12.4 us).
 template <class Factor>
 int launch_phase(int layout, unsigned log_tile, void* rho, unsigned n, const Factor& fac, cudaStream_t st) {
+    if (n <= kDirectSmall) {
+        DevMem mem{static_cast<double2*>(rho)};
+        const unsigned grid = direct_grid(2 * n);
+        if (layout == 1) k_direct_phase<<<grid, kDirectThreads, 0, st>>>(mem, PackedMap{idx_t(1) << n}, n, fac);
+        else k_direct_phase<<<grid, kDirectThreads, 0, st>>>(mem, TiledMap{idx_t(1) << n, log_tile}, n, fac);
+        return finish_launch();
+    }
     const PhaseGeom g = phase_geometry(n, layout == 2 ? log_tile : 5u);
     const unsigned grid = grid_for(phase_items_per_block(), g.items, kFullGrid);
     DevMem mem{static_cast<double2*>(rho)};

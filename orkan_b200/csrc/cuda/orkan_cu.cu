@@ -2,6 +2,7 @@
 // geometry, template dispatch, and the per-device scratch buffer used by reductions
 // and by the exp_diag phase tables.
 #include "common.cuh"
+#include "dm_direct.cuh"
 #include "dm_engine.cuh"
 #include "dm_phase.cuh"
 #include "launch.cuh"
@@ -105,6 +106,35 @@ int launch_engine_map(int layout, unsigned log_tile, void* rho, unsigned n, DmGe
     }
     return finish_launch();
 }
+
+// An operation on 2 x 2 groups over bit q.
+template <class Op>
+int launch_direct(int layout, unsigned log_tile, void* rho, unsigned n, unsigned q, const Op& op, cudaStream_t st) {
+    const DevMem mem{static_cast<double2*>(rho)};
+    const PackedMap pm{idx_t(1) << n};
+    const TiledMap tm{idx_t(1) << n, log_tile};
+    if (n <= kDirectSmall) {
+        const unsigned grid = direct_grid(2 * (n - 1));
+        if (layout == 1) k_direct_group<<<grid, kDirectThreads, 0, st>>>(mem, pm, n, q, op);
+        else k_direct_group<<<grid, kDirectThreads, 0, st>>>(mem, tm, n, q, op);
+    } else {
+        const idx_t nt = idx_t(1) << (n - 6);          // tiles of 32 groups per side
+        const unsigned grid = grid_for(1, nt * (nt + 1) / 2, kFullGrid);
+        if (layout == 1) k_direct_tile<<<grid, kDirectThreads, 0, st>>>(mem, pm, n, q, op);
+        else k_direct_tile<<<grid, kDirectThreads, 0, st>>>(mem, tm, n, q, op);
+    }
+    return finish_launch();
+}
+// Does an operation on 2 x 2 groups over bit q take the direct kernels?  All but the top qubit of large tiled
+// matrices do (14 q: 796 against 762 us there; 13 q 205 against 206), where every block's (r0, c1) tile is
+// transposed.  The engine's test hooks ask for an engine launch.
+bool direct_wins(int layout, unsigned n, unsigned q) {
+    if (g_engine_test_polls.load(std::memory_order_relaxed)) return false;
+    return layout == 1 || n < 14 || q + 1 < n;
+}
+// SWAP: one thread per element while the matrix lies in L2 (11 q: 16.5 against 22.7 us packed, 20.8 against 22.4
+// tiled; 12 q: 64 against 71, 99 against 66).
+constexpr unsigned kDirectSwap = 11;
 
 // Largest engine block side when at most one gate qubit lies above the sub-tile (a power of
 // two in [8, 64]).  Tuning knob: environment variable ORKAN_DM_MAX_V, read once.
@@ -304,6 +334,11 @@ int orkan_cu_dm_unitary(int layout, unsigned log_tile, void* rho, unsigned n, un
         return (int)cudaErrorInvalidValue;
     DmGeom g;
     if (!dm_geometry(n, k, qubits, ls_max_for(layout, log_tile), &g, dm_max_v_low())) return (int)cudaErrorInvalidValue;
+    if (k == 1 && direct_wins(layout, n, qubits[0])) {
+        DirectMix1 op;
+        for (unsigned i = 0; i < 4; ++i) op.u[i] = ld_c(u, i);
+        return launch_direct(layout, log_tile, rho, n, qubits[0], op, as_stream(stream));
+    }
     if (k == 1) {
         OpMix1 op;
         for (unsigned i = 0; i < 4; ++i) op.u[i] = ld_c(u, i);
@@ -329,6 +364,27 @@ int orkan_cu_dm_monomial(int layout, unsigned log_tile, void* rho, unsigned n, u
     DmGeom g;
     if (!dm_monomial_setup(n, k, qubits, op, ls_max_for(layout, log_tile), dm_max_v_low(), &g))
         return (int)cudaErrorInvalidValue;
+    if (op.flip && op.parity && n <= kDirectSwap && direct_wins(layout, n, 0)) {
+        const DevMem mem{static_cast<double2*>(rho)};
+        const unsigned grid = direct_grid(2 * n);
+        if (layout == 1)
+            k_direct_swap<<<grid, kDirectThreads, 0, as_stream(stream)>>>(mem, PackedMap{idx_t(1) << n}, n, qubits[0],
+                                                                          qubits[1]);
+        else
+            k_direct_swap<<<grid, kDirectThreads, 0, as_stream(stream)>>>(mem, TiledMap{idx_t(1) << n, log_tile}, n,
+                                                                          qubits[0], qubits[1]);
+        return finish_launch();
+    }
+    if (op.flip && !op.parity && direct_wins(layout, n, qubits[k - 1])) {
+        unsigned long long ctrl = 0;
+        for (unsigned j = 0; j + 1 < k; ++j) ctrl |= 1ull << qubits[j];
+        const bool unit = op.p0.x == 1.0 && op.p0.y == 0.0 && op.p1.x == 1.0 && op.p1.y == 0.0;
+        if (unit)
+            return launch_direct(layout, log_tile, rho, n, qubits[k - 1], DirectFlip<true>{ctrl, op.p0, op.p1},
+                                 as_stream(stream));
+        return launch_direct(layout, log_tile, rho, n, qubits[k - 1], DirectFlip<false>{ctrl, op.p0, op.p1},
+                             as_stream(stream));
+    }
     return launch_engine_map(layout, log_tile, rho, n, g, op, as_stream(stream));
 }
 
@@ -365,6 +421,11 @@ int orkan_cu_dm_phase(int layout, unsigned log_tile, void* rho, unsigned n, unsi
 int orkan_cu_dm_superop1(int layout, unsigned log_tile, void* rho, unsigned n, unsigned target, const double* sop,
                          void* stream) {
     if (!rho || !sop || !layout_ok(layout, log_tile) || target >= n || n > 40) return (int)cudaErrorInvalidValue;
+    if (direct_wins(layout, n, target)) {
+        DirectSuper1 d;
+        for (unsigned i = 0; i < 16; ++i) d.s[i] = ld_c(sop, i);
+        return launch_direct(layout, log_tile, rho, n, target, d, as_stream(stream));
+    }
     OpSuper1 op;
     for (unsigned i = 0; i < 16; ++i) op.s[i] = ld_c(sop, i);
     DmGeom g;

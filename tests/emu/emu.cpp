@@ -9,6 +9,7 @@
 // the storage and that each stored element is read and written exactly as often as the
 // layout's ownership rules require.  It is never used by the product library.
 #include "../../orkan_b200/csrc/cuda/common.cuh"
+#include "../../orkan_b200/csrc/cuda/dm_direct.cuh"
 #include "../../orkan_b200/csrc/cuda/dm_engine.cuh"
 #include "../../orkan_b200/csrc/cuda/dm_phase.cuh"
 #include "../../orkan_b200/csrc/cuda/pure.cuh"
@@ -374,6 +375,75 @@ int emu_dm_phase(int layout, unsigned log_tile, double* rho, uint64_t len, unsig
     for (unsigned y = 0; y < 8; ++y) fac.phase[y] = y < (1u << k) ? ldc(phase, y) : c2(1.0, 0.0);
     run_phase(layout, log_tile, mem, n, fac);
     return 0;
+}
+
+// The direct kernels (dm_direct.cuh).  op: 0 unitary (u = 4 complex), 1 superoperator (16), 2 controlled flip with
+// the qubits' last as target (p0, p1), 3 SWAP, 4 phase of a controlled diagonal gate (ph); tile != 0 takes
+// k_direct_tile (n >= 6), else one thread per group.
+}  // extern "C"
+
+namespace {
+template <class Map, class Op>
+void run_direct(const EmuMem& mem, const Map& map, unsigned n, unsigned q, const Op& op, int tile) {
+    if (!tile) {
+        for (idx_t t = 0; t < (idx_t(1) << (2 * (n - 1))); ++t) direct_small(mem, map, n, q, op, t);
+        return;
+    }
+    const idx_t nt = idx_t(1) << (n - 6);
+    std::vector<double2> sh(kDirectTile * kDirectPitch);
+    for (idx_t b = 0; b < nt * (nt + 1) / 2; ++b) {
+        const DirectWhere w = direct_where<Map>(b, n, q);
+        if (w.diag) {
+            for (unsigned e = 0; e < kDirectTile * kDirectTile; ++e) {
+                idx_t u, v;
+                direct_tile_uv<Map>(w, e % kDirectTile, e / kDirectTile, &u, &v);
+                direct_group(mem, map, q, op, u, v);
+            }
+            continue;
+        }
+        for (int phase = w.transposed ? 0 : 1; phase < (w.transposed ? 3 : 2); ++phase)
+            for (unsigned t = 0; t < kDirectThreads; ++t)
+                direct_tile_phase(phase, mem, map, q, op, w, sh.data(), t, kDirectThreads);
+    }
+}
+template <class Map>
+int run_direct_op(const EmuMem& mem, const Map& map, unsigned n, int op, unsigned k, const unsigned* q, const double* par,
+                  int tile) {
+    if (op == 0) {
+        DirectMix1 o;
+        for (unsigned i = 0; i < 4; ++i) o.u[i] = ldc(par, i);
+        run_direct(mem, map, n, q[0], o, tile);
+    } else if (op == 1) {
+        DirectSuper1 o;
+        for (unsigned i = 0; i < 16; ++i) o.s[i] = ldc(par, i);
+        run_direct(mem, map, n, q[0], o, tile);
+    } else if (op == 2) {
+        unsigned long long ctrl = 0;
+        for (unsigned j = 0; j + 1 < k; ++j) ctrl |= 1ull << q[j];
+        const double2 p0 = ldc(par, 0), p1 = ldc(par, 1);
+        if (p0.x == 1.0 && p1.x == 1.0) run_direct(mem, map, n, q[k - 1], DirectFlip<true>{ctrl, p0, p1}, tile);
+        else run_direct(mem, map, n, q[k - 1], DirectFlip<false>{ctrl, p0, p1}, tile);
+    } else if (op == 3) {
+        for (idx_t t = 0; t < (idx_t(1) << (2 * n)); ++t) direct_swap(mem, map, n, q[0], q[1], t);
+    } else {
+        GateFactorCtrl f;
+        f.mask = 0;
+        for (unsigned j = 0; j < k; ++j) f.mask |= 1ull << q[j];
+        f.ph = ldc(par, 0);
+        for (idx_t t = 0; t < (idx_t(1) << (2 * n)); ++t) direct_phase(mem, map, n, f, t);
+    }
+    return 0;
+}
+}  // namespace
+
+extern "C" {
+
+int emu_dm_direct(int layout, unsigned log_tile, double* rho, uint64_t len, unsigned n, int op, unsigned k,
+                  const unsigned* qubits, const double* par, int tile, uint32_t* reads, uint32_t* writes,
+                  uint64_t* oob) {
+    const EmuMem mem{reinterpret_cast<double2*>(rho), len, reads, writes, oob};
+    if (layout == 1) return run_direct_op(mem, PackedMap{idx_t(1) << n}, n, op, k, qubits, par, tile);
+    return run_direct_op(mem, TiledMap{idx_t(1) << n, log_tile}, n, op, k, qubits, par, tile);
 }
 
 // One chain of 1-qubit channels on ascending distinct qubits (k <= 6); -2: they do not fit one

@@ -20,7 +20,7 @@ LAYOUT = {"pure": 0, "packed": 1, "tiled": 2}
 def build() -> str:
     src = os.path.join(HERE, "emu", "emu.cpp")
     deps = [src] + [os.path.join(HERE, "..", "orkan_b200", "csrc", "cuda", f)
-                    for f in ("common.cuh", "dm_engine.cuh", "dm_phase.cuh", "pure.cuh", "pure_fused.cuh", "qaoa.cuh")]
+                    for f in ("common.cuh", "dm_direct.cuh", "dm_engine.cuh", "dm_phase.cuh", "pure.cuh", "pure_fused.cuh", "qaoa.cuh")]
     deps.append(os.path.join(HERE, "..", "include", "orkan_cu.h"))
     if not os.path.exists(LIB) or any(os.path.getmtime(d) > os.path.getmtime(LIB) for d in deps):
         import subprocess
@@ -98,6 +98,16 @@ def dm_superop1(layout, lt, data, n, target, sop):
     f = lib().emu_dm_superop1
     return _run(f, data, lambda o, r, w, b: (LAYOUT[layout], lt, _ptr(o), C.c_uint64(o.size), n, target, _ptr(s),
                                              _ptr(r), _ptr(w), C.byref(b)))
+
+
+def dm_direct(layout, lt, data, n, op, qubits, par, tile=False):
+    """The direct kernels; op: "unitary", "super", "flip", "swap" or "ctrlphase" (emu_dm_direct)."""
+    q = _arr(qubits, np.uint32)
+    s = _arr(np.asarray(par if len(par) else [0]).reshape(-1), np.complex128)
+    code = ["unitary", "super", "flip", "swap", "ctrlphase"].index(op)
+    return _run(lib().emu_dm_direct, data,
+                lambda o, r, w, b: (LAYOUT[layout], lt, _ptr(o), C.c_uint64(o.size), n, code, len(q), _ptr(q), _ptr(s),
+                                    int(tile), _ptr(r), _ptr(w), C.byref(b)))
 
 
 def dm_chain(layout, lt, data, n, qubits, sops):
