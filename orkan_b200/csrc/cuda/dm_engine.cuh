@@ -117,21 +117,22 @@ inline bool dm_geometry(unsigned n, unsigned k, const unsigned* qubits, unsigned
 }
 
 // Geometry of a chain of 1-qubit operations on the k distinct qubits of the ascending list
-// qubits: the largest sub-tile whose block, with the qubits above it as pairing bits (at most
-// 3), stays within 64 x 64.  vbit[j] receives the virtual bit of qubits[j].  False when the
-// qubits do not fit one block.
+// qubits: the largest sub-tile whose block, with the qubits above it as pairing bits (at most 2),
+// stays within 64 x 64.  vbit[j] receives the virtual bit of qubits[j].  False when the qubits do
+// not fit one block.  (With three pairing bits the lines are 128 bytes, and a bulk copy each takes as
+// long as four times that: 183 us for qubits 6-8 at 12 q, 82 us for 6-7 and 51 us for 8 alone.)
 inline bool dm_chain_geometry(unsigned n, unsigned k, const unsigned* qubits, unsigned ls_max, DmGeom* g,
                               unsigned* vbit) {
     if (k < 1 || k > 6 || n < k || qubits[k - 1] >= n) return false;
     for (int l = (int)(ls_max < n ? ls_max : n); l >= 0; --l) {
         const unsigned ls = (unsigned)l;
-        unsigned hq[3], h = 0, above = 0;
+        unsigned hq[2], h = 0, above = 0;
         for (unsigned j = 0; j < k; ++j)
             if (qubits[j] >= ls) {
-                if (above < 3) hq[above] = qubits[j];
+                if (above < 2) hq[above] = qubits[j];
                 ++above;
             }
-        if (above > 3 || ls + above > 6) continue;
+        if (above > 2 || ls + above > 6) continue;
         h = above;
         if (h == 0 && ls < n && ls + 1 <= 6) hq[h++] = ls;       // pair the sub-tiles along qubit ls
         g->d = idx_t(1) << n;
