@@ -85,6 +85,10 @@ class Orkan:
             getattr(L, g).argtypes = [P, C.c_ubyte, C.c_ubyte]
             getattr(L, g).restype = None
         L.ccx.argtypes = [P, C.c_ubyte, C.c_ubyte, C.c_ubyte]
+        L.ccx.restype = None
+        self._gates = {g: getattr(L, g) for g in ("x", "y", "z", "h", "s", "sdg", "t", "tdg", "hy", "rx", "ry", "rz", "p",
+                                                  "cx", "cy", "cz", "ccx")}
+        self._gates["swap"] = L.swap_gate
         L.state_init.argtypes = [P, C.c_ubyte, C.POINTER(vp)]
         L.state_free.argtypes = [P]
         L.state_plus.argtypes = [P, C.c_ubyte]
@@ -185,7 +189,15 @@ class Orkan:
 
     # ---- operations --------------------------------------------------------------
     def gate(self, s: StateT, name: str, qubits, theta: float | None = None) -> None:
-        fn = getattr(self.lib, "swap_gate" if name == "swap" else name)
+        fn = self._gates.get(name) or getattr(self.lib, name)
+        try:                                   # plain ints and floats need no conversion here
+            if theta is None:
+                fn(s, *qubits)
+            else:
+                fn(s, *qubits, theta)
+            return
+        except C.ArgumentError:
+            pass
         args = [C.byref(s)] + [int(q) for q in qubits]
         if theta is not None:
             args.append(float(theta))

@@ -1038,6 +1038,14 @@ inline bool monomial_is_controlled_flip(const OpMonomial& op, unsigned k) {
     return true;
 }
 
+// SWAP with unit phases.
+inline bool monomial_is_swap(const OpMonomial& op, unsigned k) {
+    if (k != 2) return false;
+    for (unsigned l = 0; l < 4; ++l)
+        if (op.src[l] != (l == 1 ? 2u : l == 2 ? 1u : l) || op.phase[l].x != 1.0 || op.phase[l].y != 0.0) return false;
+    return true;
+}
+
 // Host set-up of a monomial gate launch (geometry, fixed rows, operator form).
 //
 // A controlled flip is laid out over its target alone, so its block is as small as a
@@ -1081,15 +1089,11 @@ inline bool dm_monomial_setup(unsigned n, unsigned k, const unsigned* qubits, Op
     if (!dm_geometry(n, k, qubits, ls_max, g, max_v_low)) return false;
     g->fixmask = monomial_fixmask(op, m);
     g->fixrows = dm_fixed_rows(*g);
-    if (k == 2 && op.src[0] == 0 && op.src[1] == 2 && op.src[2] == 1 && op.src[3] == 3) {
-        bool unit = true;
-        for (unsigned l = 0; l < 4; ++l) unit = unit && op.phase[l].x == 1.0 && op.phase[l].y == 0.0;
-        if (unit) {
-            op.flip = 1;
-            op.parity = 1;
-            op.tmask = (1u << g->vbit[0]) | (1u << g->vbit[1]);
-            op.tbit = 1u << g->vbit[1];
-        }
+    if (monomial_is_swap(op, k)) {
+        op.flip = 1;
+        op.parity = 1;
+        op.tmask = (1u << g->vbit[0]) | (1u << g->vbit[1]);
+        op.tbit = 1u << g->vbit[1];
     }
     return true;
 }

@@ -151,6 +151,16 @@ unsigned dm_max_v_low() {
     return v;
 }
 
+// k distinct qubits of an n-qubit state?
+inline bool qubits_ok(unsigned n, unsigned k, const unsigned* qubits) {
+    for (unsigned j = 0; j < k; ++j) {
+        if (qubits[j] >= n) return false;
+        for (unsigned i = 0; i < j; ++i)
+            if (qubits[i] == qubits[j]) return false;
+    }
+    return true;
+}
+
 inline bool layout_ok(int layout, unsigned log_tile) {
     if (layout == 1) return true;
     if (layout == 2) return log_tile >= 1 && log_tile <= 8;
@@ -332,13 +342,14 @@ int orkan_cu_dm_unitary(int layout, unsigned log_tile, void* rho, unsigned n, un
                         const double* u, void* stream) {
     if (!rho || !qubits || !u || !layout_ok(layout, log_tile) || (k != 1 && k != 2) || n > 40)
         return (int)cudaErrorInvalidValue;
-    DmGeom g;
-    if (!dm_geometry(n, k, qubits, ls_max_for(layout, log_tile), &g, dm_max_v_low())) return (int)cudaErrorInvalidValue;
+    if (!qubits_ok(n, k, qubits)) return (int)cudaErrorInvalidValue;
     if (k == 1 && direct_wins(layout, n, qubits[0])) {
         DirectMix1 op;
         for (unsigned i = 0; i < 4; ++i) op.u[i] = ld_c(u, i);
         return launch_direct(layout, log_tile, rho, n, qubits[0], op, as_stream(stream));
     }
+    DmGeom g;
+    if (!dm_geometry(n, k, qubits, ls_max_for(layout, log_tile), &g, dm_max_v_low())) return (int)cudaErrorInvalidValue;
     if (k == 1) {
         OpMix1 op;
         for (unsigned i = 0; i < 4; ++i) op.u[i] = ld_c(u, i);
@@ -361,10 +372,8 @@ int orkan_cu_dm_monomial(int layout, unsigned log_tile, void* rho, unsigned n, u
         op.src[y] = src[y];
         op.phase[y] = ld_c(phase, y);
     }
-    DmGeom g;
-    if (!dm_monomial_setup(n, k, qubits, op, ls_max_for(layout, log_tile), dm_max_v_low(), &g))
-        return (int)cudaErrorInvalidValue;
-    if (op.flip && op.parity && n <= kDirectSwap && direct_wins(layout, n, 0)) {
+    if (!qubits_ok(n, k, qubits)) return (int)cudaErrorInvalidValue;
+    if (n <= kDirectSwap && monomial_is_swap(op, k) && direct_wins(layout, n, 0)) {
         const DevMem mem{static_cast<double2*>(rho)};
         const unsigned grid = direct_grid(2 * n);
         if (layout == 1)
@@ -375,16 +384,17 @@ int orkan_cu_dm_monomial(int layout, unsigned log_tile, void* rho, unsigned n, u
                                                                           qubits[0], qubits[1]);
         return finish_launch();
     }
-    if (op.flip && !op.parity && direct_wins(layout, n, qubits[k - 1])) {
+    if (monomial_is_controlled_flip(op, k) && direct_wins(layout, n, qubits[k - 1])) {
         unsigned long long ctrl = 0;
         for (unsigned j = 0; j + 1 < k; ++j) ctrl |= 1ull << qubits[j];
-        const bool unit = op.p0.x == 1.0 && op.p0.y == 0.0 && op.p1.x == 1.0 && op.p1.y == 0.0;
-        if (unit)
-            return launch_direct(layout, log_tile, rho, n, qubits[k - 1], DirectFlip<true>{ctrl, op.p0, op.p1},
-                                 as_stream(stream));
-        return launch_direct(layout, log_tile, rho, n, qubits[k - 1], DirectFlip<false>{ctrl, op.p0, op.p1},
-                             as_stream(stream));
+        const double2 p0 = op.phase[m - 2], p1 = op.phase[m - 1];
+        if (p0.x == 1.0 && p0.y == 0.0 && p1.x == 1.0 && p1.y == 0.0)
+            return launch_direct(layout, log_tile, rho, n, qubits[k - 1], DirectFlip<true>{ctrl, p0, p1}, as_stream(stream));
+        return launch_direct(layout, log_tile, rho, n, qubits[k - 1], DirectFlip<false>{ctrl, p0, p1}, as_stream(stream));
     }
+    DmGeom g;
+    if (!dm_monomial_setup(n, k, qubits, op, ls_max_for(layout, log_tile), dm_max_v_low(), &g))
+        return (int)cudaErrorInvalidValue;
     return launch_engine_map(layout, log_tile, rho, n, g, op, as_stream(stream));
 }
 
