@@ -163,7 +163,7 @@ struct PassShape {
 // Measured (16 instances, p = 4, ms per run) against two 256-thread blocks per SM that filled,
 // computed and stored one item after the other on the whole state: 24 qubits 5.61 against
 // 17.17, 22 qubits 1.41 against 4.13, 20 qubits 0.41 against 0.95, 16 qubits 0.086 against
-// 0.098; 8 weighted instances of 24 qubits at p = 6 6.60 against 19.8.  Half of the state's
+// 0.098; 8 weighted instances of 24 qubits at p = 6 5.89 against 19.8.  Half of the state's
 // amplitudes account for a factor of two, the staging and the shorter stages for the rest.
 template <class CostT, unsigned C>
 __global__ void __launch_bounds__(PassShape<C>::kBlock, 1)
@@ -205,6 +205,10 @@ __global__ void __launch_bounds__(PassShape<C>::kBlock, 1)
                 double2* tab = reinterpret_cast<double2*>(smem_q + L.tab + L.tab_stride * b);
                 for (unsigned e = st; e < T.tstride; e += kStageThreads)
                     QaoaDevPsi{const_cast<double2*>(row)}.cp16(tab + e, e);
+            }
+            if (!kBytes && st == 0) {                  // the item's FP64 costs on their way to L2
+                const double* src = static_cast<const double*>(I.cost) + ((size_t)(w & ((1u << P.li) - 1)) << C);
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(src), "r"(8u << C) : "memory");
             }
             if (P.layer_a >= 0)
                 qaoa_fill(P.geo, QaoaDevPsi{I.psi}, w & ((1u << P.li) - 1), reinterpret_cast<double2*>(smem_q + L.buf_stride * b),
