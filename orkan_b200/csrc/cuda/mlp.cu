@@ -24,6 +24,12 @@ __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(
 __device__ __forceinline__ float gelu_grad(float z) {
     return 0.5f * (1.0f + erff(z * kInvSqrt2)) + z * kInvSqrt2Pi * expf(-0.5f * z * z);
 }
+// Both from one erff.
+__device__ __forceinline__ void gelu_both(float z, float& act, float& slope) {
+    const float e = 1.0f + erff(z * kInvSqrt2);
+    act = 0.5f * z * e;
+    slope = 0.5f * e + z * kInvSqrt2Pi * expf(-0.5f * z * z);
+}
 
 enum Epi : int { kEpiStore = 0, kEpiBiasGelu = 1, kEpiGeluBack = 2 };
 
@@ -263,9 +269,9 @@ __global__ void k_copy_loss(const float* __restrict__ src, const unsigned* __res
 //
 // Bound: FP32 FMAs (60 us for 32768 rows at 74 TFLOP/s) for tall tiles; latency for one batch, where an
 // SM has one 8-row tile.  Measured against one tiled GEMM, row dot and column sum after the other:
-// forward of 32768 rows 131 us (32 calls of 1024 rows: 1115 us), gradients of 1024 rows 72 us with the
-// host's part (264 us), of which k_rows 28 us, k_wgrad 7.7 us and k_reduce 2.9 us, a training step of
-// 1024 rows 48 us (210 us).
+// forward of 32768 rows 131 us (32 calls of 1024 rows: 1115 us), gradients of 1024 rows 67 us with the
+// host's part (264 us), of which k_rows 21 us, k_wgrad 7.7 us and k_reduce 2.9 us, a training step of
+// 1024 rows 44 us (210 us).
 constexpr int kFH = 256, kFMaxIn = 64, kFThreads = 256, kFK = 16, kFP = 260, kFPT = 258;
 
 struct RowsArgs {
@@ -286,6 +292,11 @@ __device__ __forceinline__ unsigned long long pack2(float v) {
 }
 __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 __device__ __forceinline__ float half_of(unsigned long long v, int i) {
     return __uint_as_float((unsigned)(i ? v >> 32 : v & 0xffffffffull));
@@ -314,18 +325,87 @@ __device__ __forceinline__ void rows_mma(unsigned long long (&acc)[4][RG], const
     }
 }
 
+// An 8-row tile has one column per thread in that form, and five shared-memory wavefronts for eight FMAs a
+// lane.  There the k of a chunk are split over four groups of two warps instead, a thread takes 4 columns
+// (8 wavefronts for 32 FMAs), and the four partial sums meet in shared memory in the order of k
+// (k_rows<1, true> of 1024 rows 28.3 -> 20.8 us, with the biases and W1 fetched ahead; forward 14.6 -> 12.6 us).
+// acc[row pair][column c]: columns of the forward pass 128 half + 4 lane + c (a 16-byte load per k), of the
+// backward pass 128 half + lane + 32 c, whose W2 rows are staged as they lie, kFS floats apart (a 16-byte
+// load is four k of one column, and 8 lanes fall on all banks).
+constexpr int kFS = 20, kFSlot = 34;
+__device__ __forceinline__ void split_fma(unsigned long long (&acc)[4][4], const float* A, int c, float w) {
+    const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(A), a1 = *reinterpret_cast<const ulonglong2*>(A + 4);
+    const unsigned long long ww = pack2(w);
+    fma2(acc[0][c], a0.x, ww);
+    fma2(acc[1][c], a0.y, ww);
+    fma2(acc[2][c], a1.x, ww);
+    fma2(acc[3][c], a1.y, ww);
+}
+__device__ __forceinline__ void split_forward(unsigned long long (&acc)[4][4], const float* A, const float* W) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 w = *reinterpret_cast<const float4*>(W + k * kFP);
+        split_fma(acc, A + k * 8, 0, w.x);
+        split_fma(acc, A + k * 8, 1, w.y);
+        split_fma(acc, A + k * 8, 2, w.z);
+        split_fma(acc, A + k * 8, 3, w.w);
+    }
+}
+__device__ __forceinline__ void split_backward(unsigned long long (&acc)[4][4], const float* A, const float* W) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float4 w = *reinterpret_cast<const float4*>(W + 32 * c * kFS);
+        split_fma(acc, A, c, w.x);
+        split_fma(acc, A + 8, c, w.y);
+        split_fma(acc, A + 16, c, w.z);
+        split_fma(acc, A + 24, c, w.w);
+    }
+}
+// The sums over the four groups, for column tid: slot (half, c) starts at 34 (4 half + c) and holds one
+// 16-byte element per lane, so that the reads of either column order are free of conflicts.
+template <bool FWD>
+__device__ __forceinline__ void split_sum(const unsigned long long (&acc)[4][4], float* P, unsigned long long (&out)[4][1]) {
+    const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
+    ulonglong2* B = reinterpret_cast<ulonglong2*>(P);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            B[(warp / 2 * 2 + q) * 8 * kFSlot + (warp % 2 * 4 + c) * kFSlot + lane] =
+                make_ulonglong2(acc[2 * q][c], acc[2 * q + 1][c]);
+    __syncthreads();
+    const int slot = FWD ? (tid / 128 * 4 + tid % 4) * kFSlot + tid % 128 / 4 : tid / 32 * kFSlot + tid % 32;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        ulonglong2 s = B[q * 8 * kFSlot + slot];
+#pragma unroll
+        for (int g = 1; g < 4; ++g) {
+            const ulonglong2 v = B[(2 * g + q) * 8 * kFSlot + slot];
+            s.x = add2(s.x, v.x);
+            s.y = add2(s.y, v.y);
+        }
+        out[2 * q][0] = s.x;
+        out[2 * q + 1][0] = s.y;
+    }
+}
+
+// W2 chunks in shared memory: three for the 8-row tiles (two of them on their way), else two.
+template <int RG>
+constexpr int kFChunk = RG == 1 ? kFH * kFS : kFK * kFP;
+template <int RG>
+constexpr int kFChunks = RG == 1 ? 3 : 2;
 template <int RG>
 size_t rows_smem(int n_in) {
-    return sizeof(float) * (size_t)(kFP * 8 * RG + 2 * kFK * kFP + n_in * 8 * RG + 64 + 16 * RG);
+    return sizeof(float) * (size_t)(kFP * 8 * RG + kFChunks<RG> * kFChunk<RG> + n_in * 8 * RG + 64 + 16 * RG);
 }
 
 template <int RG, bool BWD>
 __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const RowsArgs a) {
-    constexpr int BM = 8 * RG, CG = 8 / RG;
+    constexpr int BM = 8 * RG, CG = 8 / RG, NC = kFChunks<RG>, kW = kFChunk<RG>, kChunks = kFH / kFK;
     extern __shared__ __align__(16) float fsm[];
     float* As = fsm;                                   // [256][BM]; later dz1 as [BM][260]
-    float* Ws = As + kFP * BM;                         // two chunks of kFK rows
-    float* Xs = Ws + 2 * kFK * kFP;                    // [n_in][BM]
+    float* Ws = As + kFP * BM;                         // NC chunks of kFK rows
+    float* Xs = Ws + NC * kW;                    // [n_in][BM]
     float* red = Xs + a.n_in * BM;                     // [8 warps][8 rows]
     float* dys = red + 64;                             // [BM]
     float* errs = dys + BM;                            // [BM]
@@ -336,18 +416,27 @@ __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int e = tid + kFThreads * i, r = e / 64, c = (e % 64) * 4;
-            cp_async16(Ws + buf * kFK * kFP + r * kFP + c, a.W2 + (size_t)(kc * kFK + r) * kFH + c);
+            cp_async16(Ws + buf * kW + r * kFP + c, a.W2 + (size_t)(kc * kFK + r) * kFH + c);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    load_w2(0, 0);
+    auto load_w2t = [&](int kc, int buf) {             // columns 16 kc .. + 15 of W2, row by row
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int e = tid + kFThreads * i;
+            cp_async16(Ws + buf * kW + e / 4 * kFS + e % 4 * 4, a.W2 + (size_t)(e / 4) * kFH + kc * kFK + e % 4 * 4);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+#pragma unroll
+    for (int c = 0; c + 1 < NC; ++c) load_w2(c, c);
     for (int e = tid; e < a.n_in * BM; e += kFThreads) {
         const int r = e / a.n_in, k = e % a.n_in;
         Xs[k * BM + r] = row0 + r < a.rows ? a.x[(size_t)(row0 + r) * a.n_in + k] : 0.f;
     }
     __syncthreads();
     unsigned long long acc[4][RG];
-    float z1[BWD ? 8 : 1][RG];
+    float d1[BWD ? 8 : 1][RG];                         // gelu'(z1)
     auto clear = [&] {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -355,6 +444,7 @@ __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const
             for (int c = 0; c < RG; ++c) acc[i][c] = 0ull;
     };
     clear();
+#pragma unroll 4
     for (int k = 0; k < a.n_in; ++k) {
         const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(Xs + k * BM + rg * 8);
         const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(Xs + k * BM + rg * 8 + 4);
@@ -375,19 +465,36 @@ __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
             const float z = half_of(acc[r / 2][c], r % 2) + bias;
-            if (BWD) z1[r][c] = z;
-            v[r] = gelu(z);
+            if (BWD) gelu_both(z, v[r], d1[r][c]);
+            else v[r] = gelu(z);
             if (BWD && a.A1 && my0 + r < a.rows) a.A1[(size_t)(my0 + r) * kFH + col] = v[r];
         }
         *reinterpret_cast<float4*>(As + col * BM + rg * 8) = make_float4(v[0], v[1], v[2], v[3]);
         *reinterpret_cast<float4*>(As + col * BM + rg * 8 + 4) = make_float4(v[4], v[5], v[6], v[7]);
     }
     clear();
-    for (int kc = 0; kc < kFH / kFK; ++kc) {
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();                               // the chunk is in, the other buffer is read
-        if (kc + 1 < kFH / kFK) load_w2(kc + 1, (kc + 1) & 1);
-        rows_mma<RG>(acc, As + kc * kFK * BM + rg * 8, Ws + (kc & 1) * kFK * kFP + col0, kFP);
+    // one column per thread: its bias and output weight arrive under the product
+    const float bias2 = RG == 1 ? __ldg(a.b2 + col0) : 0.f, out3 = RG == 1 ? __ldg(a.w3 + col0) : 0.f;
+    const int kg = warp / 2 * 4;                       // 8-row tiles: this warp's k of a chunk, and its columns
+    // every chunk by mma(its index, its buffer), the next NC - 1 on their way
+    auto chunks = [&](auto& load, auto mma) {
+        for (int kc = 0; kc < kChunks; ++kc) {
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(NC - 2) : "memory");
+            __syncthreads();                           // the chunk is in, the one before it is read
+            if (kc + NC - 1 < kChunks) load(kc + NC - 1, (kc + NC - 1) % NC);
+            else if (NC > 2) asm volatile("cp.async.commit_group;\n" ::: "memory");
+            mma(kc, Ws + kc % NC * kW);
+        }
+    };
+    if constexpr (RG == 1) {
+        unsigned long long part[4][4] = {};
+        chunks(load_w2, [&](int kc, const float* W) {
+            split_forward(part, As + (kc * kFK + kg) * 8, W + kg * kFP + warp % 2 * 128 + lane * 4);
+        });
+        __syncthreads();
+        split_sum<true>(part, Ws, acc);
+    } else {
+        chunks(load_w2, [&](int kc, const float* W) { rows_mma<RG>(acc, As + kc * kFK * BM + rg * 8, W + col0, kFP); });
     }
     // z2 = acc + b2; y = gelu(z2) . w3 + b3, over the lanes by a fixed tree, then over the warps
     float p[8];
@@ -395,7 +502,7 @@ __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const
     for (int r = 0; r < 8; ++r) p[r] = 0.f;
 #pragma unroll
     for (int c = 0; c < RG; ++c) {
-        const float bias = __ldg(a.b2 + col0 + 32 * c), w3 = __ldg(a.w3 + col0 + 32 * c);
+        const float bias = RG == 1 ? bias2 : __ldg(a.b2 + col0 + 32 * c), w3 = RG == 1 ? out3 : __ldg(a.w3 + col0 + 32 * c);
 #pragma unroll
         for (int r = 0; r < 8; ++r) p[r] = fmaf(gelu(half_of(acc[r / 2][c], r % 2) + bias), w3, p[r]);
     }
@@ -419,6 +526,10 @@ __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const
         }
     }
     if constexpr (BWD) {
+        if constexpr (RG == 1) {
+#pragma unroll
+            for (int c = 0; c + 1 < NC; ++c) load_w2t(c, c);
+        }
         __syncthreads();
         if (tid == 0 && a.rowp) {
             float loss = 0.f, db3 = 0.f;
@@ -433,13 +544,15 @@ __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const
 #pragma unroll
         for (int c = 0; c < RG; ++c) {
             const int col = col0 + 32 * c;
-            const float bias = __ldg(a.b2 + col), w3 = __ldg(a.w3 + col);
+            const float bias = RG == 1 ? bias2 : __ldg(a.b2 + col), w3 = RG == 1 ? out3 : __ldg(a.w3 + col);
             float v[8], dw3 = 0.f, db2 = 0.f;
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
                 const float z = half_of(acc[r / 2][c], r % 2) + bias, dy = dys[rg * 8 + r];
-                dw3 = fmaf(gelu(z), dy, dw3);
-                v[r] = dy * w3 * gelu_grad(z);
+                float act, slope;
+                gelu_both(z, act, slope);
+                dw3 = fmaf(act, dy, dw3);
+                v[r] = dy * w3 * slope;
                 db2 += v[r];
                 if (a.dZ2 && my0 + r < a.rows) a.dZ2[(size_t)(my0 + r) * kFH + col] = v[r];
             }
@@ -450,36 +563,46 @@ __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const
             *reinterpret_cast<float4*>(As + col * BM + rg * 8) = make_float4(v[0], v[1], v[2], v[3]);
             *reinterpret_cast<float4*>(As + col * BM + rg * 8 + 4) = make_float4(v[4], v[5], v[6], v[7]);
         }
-        // dz1 = (dz2 W2^T) gelu'(z1): chunk kc holds W2[:][16 kc .. + 15] transposed (pitch 258: the
-        // stores of a warp, 8 rows x 4 k, fall on 32 banks)
-        float4 w[4];
-        auto get_t = [&](int kc) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int e = tid + kFThreads * i;
-                w[i] = __ldg(reinterpret_cast<const float4*>(a.W2 + (size_t)(e / 4) * kFH + kc * kFK + (e % 4) * 4));
-            }
-        };
-        auto put_t = [&](int buf) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int e = tid + kFThreads * i;
-                float* d = Ws + buf * kFK * kFP + (e % 4) * 4 * kFPT + e / 4;
-                d[0] = w[i].x;
-                d[kFPT] = w[i].y;
-                d[2 * kFPT] = w[i].z;
-                d[3 * kFPT] = w[i].w;
-            }
-        };
-        get_t(0);
-        put_t(0);
-        clear();
-        __syncthreads();
-        for (int kc = 0; kc < kFH / kFK; ++kc) {
-            if (kc + 1 < kFH / kFK) get_t(kc + 1);
-            rows_mma<RG>(acc, As + kc * kFK * BM + rg * 8, Ws + (kc & 1) * kFK * kFP + col0, kFPT);
-            if (kc + 1 < kFH / kFK) put_t((kc + 1) & 1);
+        // dz1 = (dz2 W2^T) gelu'(z1)
+        if constexpr (RG == 1) {
+            unsigned long long part[4][4] = {};
+            chunks(load_w2t, [&](int kc, const float* W) {
+                split_backward(part, As + (kc * kFK + kg) * 8, W + (warp % 2 * 128 + lane) * kFS + kg);
+            });
             __syncthreads();
+            split_sum<false>(part, Ws, acc);
+        } else {
+            // chunk kc holds W2[:][16 kc .. + 15] transposed (pitch 258: the stores of a warp, 8 rows x 4 k,
+            // fall on 32 banks)
+            float4 w[4];
+            auto get_t = [&](int kc) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int e = tid + kFThreads * i;
+                    w[i] = __ldg(reinterpret_cast<const float4*>(a.W2 + (size_t)(e / 4) * kFH + kc * kFK + (e % 4) * 4));
+                }
+            };
+            auto put_t = [&](int buf) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int e = tid + kFThreads * i;
+                    float* d = Ws + buf * kW + (e % 4) * 4 * kFPT + e / 4;
+                    d[0] = w[i].x;
+                    d[kFPT] = w[i].y;
+                    d[2 * kFPT] = w[i].z;
+                    d[3 * kFPT] = w[i].w;
+                }
+            };
+            get_t(0);
+            put_t(0);
+            clear();
+            __syncthreads();
+            for (int kc = 0; kc < kFH / kFK; ++kc) {
+                if (kc + 1 < kFH / kFK) get_t(kc + 1);
+                rows_mma<RG>(acc, As + kc * kFK * BM + rg * 8, Ws + (kc & 1) * kW + col0, kFPT);
+                if (kc + 1 < kFH / kFK) put_t((kc + 1) & 1);
+                __syncthreads();
+            }
         }
 #pragma unroll
         for (int c = 0; c < RG; ++c) {
@@ -487,7 +610,7 @@ __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const
             float db1 = 0.f;
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
-                const float v = half_of(acc[r / 2][c], r % 2) * gelu_grad(z1[r][c]);
+                const float v = half_of(acc[r / 2][c], r % 2) * d1[r][c];
                 db1 += v;
                 if (a.dZ1 && my0 + r < a.rows) a.dZ1[(size_t)(my0 + r) * kFH + col] = v;
                 if (a.gx) As[(rg * 8 + r) * kFP + col] = v;
@@ -496,14 +619,19 @@ __global__ void __launch_bounds__(kFThreads, BWD && RG > 1 ? 1 : 2) k_rows(const
         }
         if (!a.gx) return;
         __syncthreads();
-        for (int o = warp; o < BM * a.n_in; o += kFThreads / 32) {     // dL/dx[r][k], one warp each
-            const int r = o / a.n_in, k = o % a.n_in;
-            float s = 0.f;
+        for (int r = warp; r < BM; r += kFThreads / 32) {              // dL/dx[r], one warp each
+            float dz[kFH / 32];
 #pragma unroll
-            for (int i = 0; i < kFH / 32; ++i) s = fmaf(As[r * kFP + lane + 32 * i], __ldg(a.W1 + k * kFH + lane + 32 * i), s);
+            for (int i = 0; i < kFH / 32; ++i) dz[i] = As[r * kFP + lane + 32 * i];
+#pragma unroll 4
+            for (int k = 0; k < a.n_in; ++k) {
+                float s = 0.f;
 #pragma unroll
-            for (int q = 16; q > 0; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
-            if (lane == 0 && row0 + r < a.rows) a.gx[(size_t)(row0 + r) * a.n_in + k] = s;
+                for (int i = 0; i < kFH / 32; ++i) s = fmaf(dz[i], __ldg(a.W1 + k * kFH + lane + 32 * i), s);
+#pragma unroll
+                for (int q = 16; q > 0; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
+                if (lane == 0 && row0 + r < a.rows) a.gx[(size_t)(row0 + r) * a.n_in + k] = s;
+            }
         }
     }
 }
@@ -734,14 +862,16 @@ int rows_prepare() {
     auto allow = [](const void* f, size_t bytes) {
         return (int)cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
-    int rc = allow((const void*)k_rows<4, true>, rows_smem<4>(kFMaxIn));
+    int rc = allow((const void*)k_rows<1, true>, rows_smem<1>(kFMaxIn));
+    if (!rc) rc = allow((const void*)k_rows<1, false>, rows_smem<1>(kFMaxIn));
+    if (!rc) rc = allow((const void*)k_rows<4, true>, rows_smem<4>(kFMaxIn));
     if (!rc) rc = allow((const void*)k_rows<4, false>, rows_smem<4>(kFMaxIn));
     if (!rc) rc = allow((const void*)k_rows<8, false>, rows_smem<8>(kFMaxIn));
     return rc;
 }
 
-// Rows per tile: 8 while that leaves at most two tiles per SM (measured 22.8 us for 2368 rows forward
-// and 22.9 us with 32-row tiles at 2400), then 32 (with backward z1 stays in registers as well), and
+// Rows per tile: 8 while that leaves at most two tiles per SM (measured 18.7 us for 2368 rows forward
+// and 23.1 us with 32-row tiles at 2400), then 32 (with backward z1 stays in registers as well), and
 // forward 64 once they fill two tiles per SM: 131 us for 32768 rows and 3.3 ns a row beyond, 4.1 ns
 // in 32-row tiles.
 int rows_tile(int rows, bool bwd) {
