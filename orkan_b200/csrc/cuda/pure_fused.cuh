@@ -77,6 +77,7 @@ struct FusedPlan {
     unsigned char nlq[32];     // global position of chunk id bit i (the first 32)
     unsigned K;                // qubits of a stage's group
     unsigned nstages;
+    bool din, dout;            // the first stage reads HBM, the last one writes HBM: fused_direct
     FStage st[kFuseMaxGates + 1];    // st[nstages].first = ngates
     FGate g[kFuseMaxGates];
     ORKAN_HD unsigned chunk() const { return 1u << C; }
@@ -102,6 +103,16 @@ inline unsigned long long fused_need(const orkan_fgate_t& q) {
 
 inline unsigned fused_arity(int op) {
     return op < ORKAN_FOP_CX ? 1u : (op == ORKAN_FOP_CCX ? 3u : 2u);
+}
+
+// A stage moves its amplitudes between HBM and registers itself, without the shared memory, where its
+// group leaves the lowest three qubits to the lanes: 8 lanes then have the 128 bytes of a line.  Not
+// where one block holds the state: it has no other block to wait behind, and all its copies to shared memory in
+// flight at once (200 gates at 12 qubits 162 us; 165 us with direct stages).
+inline bool fused_direct(const FusedPlan& P, const FStage& st) {
+    for (unsigned i = 0; i < P.K; ++i)
+        if (st.g[i] < 3) return false;
+    return P.C >= P.K + 3 && P.C < P.n;
 }
 
 // Build the plan of a run on an n-qubit statevector with chunks of 2^C amplitudes.  False
@@ -136,11 +147,11 @@ inline bool fused_plan(unsigned n, unsigned C, unsigned ngates, const orkan_fgat
     const unsigned most = C == n ? 3u : kFuseGroup;
     P->K = C < most ? C : most;
     // stages: consecutive gates whose mixed local bits fit a group of K bits; a group with fewer is
-    // filled with the lowest other local bits
+    // filled with the highest other local bits for the sake of fused_direct, or the lowest
     P->nstages = 0;
     unsigned cur = 0;
     auto close = [&](unsigned first, unsigned last) {
-        for (unsigned b = 0; b < C && popc64(cur) < P->K; ++b) cur |= 1u << b;
+        for (unsigned b = 0; b < C && popc64(cur) < P->K; ++b) cur |= 1u << (C < n ? C - 1 - b : b);
         FStage& st = P->st[P->nstages++];
         st.first = (unsigned char)first;
         unsigned k = 0, e[kFuseMaxLog] = {};             // element bit of a local bit of the group
@@ -232,6 +243,8 @@ inline bool fused_plan(unsigned n, unsigned C, unsigned ngates, const orkan_fgat
     }
     close(first, ngates);
     P->st[P->nstages].first = (unsigned char)ngates;
+    P->din = fused_direct(*P, P->st[0]);
+    P->dout = fused_direct(*P, P->st[P->nstages - 1]);
     return true;
 }
 
@@ -271,51 +284,67 @@ ORKAN_HD idx_t fused_off(const FusedPlan& P, unsigned j) {
     return o;
 }
 
-// A thread's share of a chunk for load and store: the 2^K amplitudes j = tid | u << (C - K), whose
-// offsets and slots are those of tid with the bits of u added, so that an amplitude costs a few
-// logic instructions.  Mem::cp16(dst, x) copies amplitude x (asynchronously on the GPU).
-struct FusedWalk {
-    idx_t off;                 // fused_off(tid)
-    unsigned slot;             // fused_phys(tid)
-    bool live;                 // tid names a share
-};
-ORKAN_HD FusedWalk fused_walk(const FusedPlan& P, unsigned tid) {
-    FusedWalk w;
-    w.live = tid < P.sets();
-    w.off = fused_off(P, tid);
-    w.slot = fused_phys(tid);
-    return w;
-}
-template <int K, class F>
-ORKAN_HD void fused_each(const FusedPlan& P, const FusedWalk& w, const F& f) {
-    if (!w.live) return;
-    idx_t go[K];
-    unsigned so[K];
+// Chunk index of set r's element 0 in a stage.
+template <int K>
+ORKAN_HD unsigned fused_set(const FusedPlan& P, const FStage& st, unsigned r) {
+    unsigned sb = 0;
 #pragma unroll
-    for (int b = 0; b < K; ++b) {
-        go[b] = idx_t(1) << P.lq[P.C - K + b];
-        so[b] = fused_phys(1u << (P.C - K + b));
-    }
+    for (unsigned i = 0; i < kFuseMaxLog - K; ++i)
+        if (i < P.C - K) sb |= ((r >> i) & 1u) << st.f[i];
+    return sb;
+}
+
+// A thread's share of a chunk for load and store.  Through the shared memory: the 2^K amplitudes
+// j = tid | u << (C - K), whose offsets and slots are those of tid with the bits of u added, so that an
+// amplitude costs a few logic instructions.  Directly: the set of the stage.
+struct FusedWalk {
+    idx_t in, out;             // global offset of the share's amplitude 0
+};
+template <int K>
+ORKAN_HD FusedWalk fused_walk(const FusedPlan& P, unsigned tid) {
+    return {fused_off(P, P.din ? fused_set<K>(P, P.st[0], tid) : tid),
+            fused_off(P, P.dout ? fused_set<K>(P, P.st[P.nstages - 1], tid) : tid)};
+}
+// f(u, global offset) of the 2^K elements whose bit b lies at local bit l(b).
+template <int K, class L, class F>
+ORKAN_HD void fused_spread(const FusedPlan& P, idx_t off, const L& l, const F& f) {
+    idx_t go[K];
+#pragma unroll
+    for (int b = 0; b < K; ++b) go[b] = idx_t(1) << P.lq[l(b)];
 #pragma unroll
     for (int u = 0; u < (1 << K); ++u) {
-        idx_t o = w.off;
-        unsigned s = w.slot;
+        idx_t o = off;
 #pragma unroll
         for (int b = 0; b < K; ++b)
-            if ((u >> b) & 1) {
-                o |= go[b];
-                s ^= so[b];
-            }
-        f(o, s);
+            if ((u >> b) & 1) o |= go[b];
+        f(u, o);
     }
 }
+// f(global offset, slot) of the share that goes through the shared memory.
+template <int K, class F>
+ORKAN_HD void fused_each(const FusedPlan& P, idx_t off, unsigned tid, const F& f) {
+    if (tid >= P.sets()) return;
+    const unsigned slot = fused_phys(tid);
+    unsigned so[K];
+#pragma unroll
+    for (int b = 0; b < K; ++b) so[b] = fused_phys(1u << (P.C - K + b));
+    fused_spread<K>(P, off, [&](int b) { return P.C - K + b; }, [&](int u, idx_t o) {
+        unsigned s = slot;
+#pragma unroll
+        for (int b = 0; b < K; ++b)
+            if ((u >> b) & 1) s ^= so[b];
+        f(o, s);
+    });
+}
+// Mem::cp16(dst, x) copies amplitude x (asynchronously on the GPU).
 template <int K, class Mem>
-ORKAN_HD void fused_load(const Mem& mem, const FusedPlan& P, const FusedWalk& w, idx_t base, double2* buf) {
-    fused_each<K>(P, w, [&](idx_t o, unsigned s) { mem.cp16(buf + s, base | o); });
+ORKAN_HD void fused_load(const Mem& mem, const FusedPlan& P, const FusedWalk& w, unsigned tid, idx_t base, double2* buf) {
+    fused_each<K>(P, w.in, tid, [&](idx_t o, unsigned s) { mem.cp16(buf + s, base | o); });
 }
 template <int K, class Mem>
-ORKAN_HD void fused_store(const Mem& mem, const FusedPlan& P, const FusedWalk& w, idx_t base, const double2* buf) {
-    fused_each<K>(P, w, [&](idx_t o, unsigned s) { mem.st(base | o, buf[s]); });
+ORKAN_HD void fused_store(const Mem& mem, const FusedPlan& P, const FusedWalk& w, unsigned tid, idx_t base,
+                          const double2* buf) {
+    fused_each<K>(P, w.out, tid, [&](idx_t o, unsigned s) { mem.st(base | o, buf[s]); });
 }
 
 // ---- register stages -------------------------------------------------------------------
@@ -446,24 +475,22 @@ ORKAN_HD void fused_apply(const FGate& g, double2 (&v)[NV], unsigned sb, idx_t b
     }
 }
 
-// Stage s of the run on the staged chunk (all threads of the block; a barrier follows).
+// Stage s of the run on a chunk (all threads of the block; a barrier follows).
 // Thread tid takes set tid: the set's 2^K amplitudes go to registers, every gate of the stage
-// whose chunk condition holds is applied, and they go back.  The swizzle is
+// whose chunk condition holds is applied, and they go back; the first stage reads HBM and the last
+// one writes it where they are direct.  The swizzle is
 // linear over disjoint bits, so element j lies at phys(sb) ^ phys(its group bits).
-template <int K>
-ORKAN_HD void fused_stage_k(const FusedPlan& P, unsigned s, idx_t base, double2* buf, unsigned r) {
+template <int K, class Mem>
+ORKAN_HD void fused_stage_k(const Mem& mem, const FusedPlan& P, const FusedWalk& w, unsigned s, idx_t base, double2* buf,
+                            unsigned r) {
     constexpr int NV = 1 << K;
     const FStage& st = P.st[s];
-    const unsigned g0 = st.first, g1 = P.st[s + 1].first, nf = P.C - K;
+    const unsigned g0 = st.first, g1 = P.st[s + 1].first;
     unsigned ph[K];
 #pragma unroll
     for (int b = 0; b < K; ++b) ph[b] = fused_phys(1u << st.g[b]) * 16u;
     if (r >= P.sets()) return;
-    unsigned sb = 0;
-#pragma unroll
-    for (unsigned i = 0; i < kFuseMaxLog - K; ++i)
-        if (i < nf) sb |= ((r >> i) & 1u) << st.f[i];
-    const unsigned psb = fused_phys(sb) * 16u;
+    const unsigned sb = fused_set<K>(P, st, r), psb = fused_phys(sb) * 16u;
     unsigned char* raw = reinterpret_cast<unsigned char*>(buf);
     auto at = [&](int j) -> double2& {
         unsigned a = psb;
@@ -472,15 +499,24 @@ ORKAN_HD void fused_stage_k(const FusedPlan& P, unsigned s, idx_t base, double2*
             if ((j >> b) & 1) a ^= ph[b];
         return *reinterpret_cast<double2*>(raw + a);
     };
+    auto bit = [&](int b) { return (unsigned)st.g[b]; };
     double2 v[NV];
+    if (s == 0 && P.din) {
+        fused_spread<K>(P, base | w.in, bit, [&](int j, idx_t o) { v[j] = mem.ld(o); });
+    } else {
 #pragma unroll
-    for (int j = 0; j < NV; ++j) v[j] = at(j);
+        for (int j = 0; j < NV; ++j) v[j] = at(j);
+    }
 #ifdef __CUDA_ARCH__
 #pragma unroll 1
 #endif
     for (unsigned gi = g0; gi < g1; ++gi) fused_apply(P.g[gi], v, sb, base);
+    if (s + 1 == P.nstages && P.dout) {
+        fused_spread<K>(P, base | w.out, bit, [&](int j, idx_t o) { mem.st(o, v[j]); });
+    } else {
 #pragma unroll
-    for (int j = 0; j < NV; ++j) at(j) = v[j];
+        for (int j = 0; j < NV; ++j) at(j) = v[j];
+    }
 }
 
 // Shared memory of one block: the chunk.
@@ -492,6 +528,7 @@ inline unsigned fused_threads(const FusedPlan& P) { return P.sets() < 32 ? 32u :
 #ifdef __CUDACC__
 struct FusedDevMem {
     double2* p;
+    __device__ __forceinline__ double2 ld(idx_t i) const { return p[i]; }
     __device__ __forceinline__ void st(idx_t i, double2 v) const { p[i] = v; }
     __device__ __forceinline__ void cp16(double2* dst, idx_t i) const {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
@@ -502,28 +539,36 @@ struct FusedDevMem {
 // Persistent blocks walk the chunks; every gate whose chunk condition holds is applied in
 // shared memory between one load and one store of the chunk.
 //
-// Bound: instruction issue.  A chunk's load, store and one stage take 26 instructions per amplitude, a
-// gate 3 to 10 (the arithmetic of an H is 4), a further stage 5; HBM takes 5.3 ms of the 9.3 ms that a run
-// of 15 random gates takes at 30 qubits (15.1 ms with 8-amplitude sets whose gates copied registers).
-// 200 random gates: 30 qubits 124.7 ms (208.7 before), 12 qubits, one block, 117 us on the GPU (277).
+// Bound: instructions and their latency at 4 warps per scheduler (128 registers: 16 amplitudes); 45 % of the
+// issue slots are used, 18 % of FP64, a third of HBM.  At 28 qubits HBM takes 1.32 ms of a run, 8 gates of one
+// stage hide under it (1.39 ms), 16 H take 1.89 ms, further ones 80 us each.  200 random gates: 30 qubits
+// 208.7 ms with 8-amplitude sets whose gates copied registers, 124.7 ms with 16-amplitude sets, 122 ms
+// with direct stages (both measured side by side: 125.9 and 122.3); 12 qubits, one block, 117 us on the GPU (277).  Fetching the next chunk to L2 ahead
+// and letting half of the blocks start later gave nothing; chunks of 2^12 save a fifth of the runs but leave two
+// blocks per SM (118.4 against 116.9 ms for 192 gates).
 template <int K>
 __global__ void __launch_bounds__(K == 4 ? 256 : kFuseThreads, K == 4 ? 2 : 1)
     k_pure_fused(FusedDevMem mem, const __grid_constant__ FusedPlan P) {
     extern __shared__ __align__(128) double2 fbuf[];
     const unsigned tid = threadIdx.x;
-    const FusedWalk w = fused_walk(P, tid);
+    const FusedWalk w = fused_walk<K>(P, tid);
     const idx_t nch = P.nchunks();
+    const bool alone = P.nstages == 1 && P.din && P.dout;    // the chunk never meets the shared memory
     for (idx_t ch = blockIdx.x; ch < nch; ch += gridDim.x) {
         const idx_t base = fused_base(P, ch);
-        fused_load<K>(mem, P, w, base, fbuf);
-        asm volatile("cp.async.wait_all;\n" ::: "memory");
-        __syncthreads();
-        for (unsigned st = 0; st < P.nstages; ++st) {
-            fused_stage_k<K>(P, st, base, fbuf, tid);
+        if (!P.din) {
+            fused_load<K>(mem, P, w, tid, base, fbuf);
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
             __syncthreads();
         }
-        fused_store<K>(mem, P, w, base, fbuf);
-        __syncthreads();
+        for (unsigned st = 0; st < P.nstages; ++st) {
+            fused_stage_k<K>(mem, P, w, st, base, fbuf, tid);
+            if (!alone) __syncthreads();
+        }
+        if (!P.dout) {
+            fused_store<K>(mem, P, w, tid, base, fbuf);
+            __syncthreads();
+        }
     }
 }
 #endif

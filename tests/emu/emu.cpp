@@ -562,10 +562,10 @@ void run_fused(const EmuMem& mem, const FusedPlan& P, unsigned grid_cap) {
     for (unsigned b = 0; b < grid; ++b)
         for (idx_t ch = b; ch < nch; ch += grid) {
             const idx_t base = fused_base(P, ch);
-            for (unsigned t = 0; t < nthr; ++t) fused_load<K>(mem, P, fused_walk(P, t), base, buf.data());
+            for (unsigned t = 0; t < nthr && !P.din; ++t) fused_load<K>(mem, P, fused_walk<K>(P, t), t, base, buf.data());
             for (unsigned st = 0; st < P.nstages; ++st)
-                for (unsigned t = 0; t < nthr; ++t) fused_stage_k<K>(P, st, base, buf.data(), t);
-            for (unsigned t = 0; t < nthr; ++t) fused_store<K>(mem, P, fused_walk(P, t), base, buf.data());
+                for (unsigned t = 0; t < nthr; ++t) fused_stage_k<K>(mem, P, fused_walk<K>(P, t), st, base, buf.data(), t);
+            for (unsigned t = 0; t < nthr && !P.dout; ++t) fused_store<K>(mem, P, fused_walk<K>(P, t), t, base, buf.data());
         }
 }
 }  // namespace
