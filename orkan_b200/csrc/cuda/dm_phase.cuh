@@ -214,7 +214,53 @@ ORKAN_HD void dm_phase_item(const Mem& mem, const Map& map, const PhaseGeom& g, 
     }
 }
 
+// A 1-qubit diagonal gate on packed storage, column by column in storage order.  Columns c and d - 1 - c
+// make one line of d positions: position p > c is row p of column c, p < c row d - 1 - p of the other, so
+// every line has the same work and both halves are contiguous.  In both halves the positions whose bit q
+// differs from c's change, and only those are numbered: h with that bit inserted.
+//
+// Bound: HBM (14 qubits: 1.07 GB each way are 330 us; for q < 1 every sector is touched, 660 us).  Against the
+// 32 x 32 items, whose lines are 512 bytes at any alignment and lie far apart: 14 qubits, q = 0 / 3 / 6 / 13
+// 647 / 558 / 383 / 325 us (757 / 672 / 425 / 379), 12 qubits 44 .. 19 us (48 .. 21), 11 qubits 12 .. 8 us (13 .. 10).
+// Controlled phases change 3/8 of the elements or fewer and stay with the items, which skip more of the
+// others (CZ on qubits 5 and 9 of 14: 328 us; 426 us by columns).
+constexpr unsigned kColThreads = 256, kColEpt = 4, kColBlock = 2048;
+
+inline idx_t phase_column_blocks(unsigned n) {           // 1 <= n
+    const idx_t half = idx_t(1) << (n - 1);
+    return half * ((half + kColBlock - 1) / kColBlock);
+}
+template <class Mem>
+ORKAN_HD void dm_phase_columns(const Mem& mem, const PackedMap& map, const GateFactor1& fac, idx_t block, unsigned tid) {
+    const idx_t d = map.d, half = d / 2, parts = (half + kColBlock - 1) / kColBlock;
+    const idx_t c = block / parts, c2nd = d - 1 - c, h0 = block % parts * kColBlock;
+    const idx_t first = map.at(c, c) - c, second = map.at(c2nd, c2nd) - c2nd;   // + row
+    const idx_t end = h0 + kColBlock < half ? h0 + kColBlock : half, bit = ~c & (idx_t(1) << fac.q);
+    for (idx_t h = h0 + tid; h < end; h += kColThreads * kColEpt) {
+        idx_t addr[kColEpt];
+        double2 val[kColEpt], f[kColEpt];
+#pragma unroll
+        for (unsigned k = 0; k < kColEpt; ++k) {
+            if (h + k * kColThreads >= end) continue;
+            const idx_t x = insert0(h + k * kColThreads, fac.q) | bit;
+            const bool one = x > c;
+            const idx_t r = one ? x : d - 1 - x;
+            fac.factor(r, one ? c : c2nd, &f[k]);
+            addr[k] = (one ? first : second) + r;
+            val[k] = mem.ld(addr[k]);
+        }
+#pragma unroll
+        for (unsigned k = 0; k < kColEpt; ++k)
+            if (h + k * kColThreads < end) mem.st(addr[k], phase_apply(f[k], val[k]));
+    }
+}
+
 #ifdef __CUDACC__
+template <class Map>
+__global__ void __launch_bounds__(kColThreads) k_dm_phase_columns(DevMem mem, Map map, GateFactor1 fac) {
+    dm_phase_columns(mem, map, fac, blockIdx.x, threadIdx.x);
+}
+
 template <class Map, class Factor>
 __global__ void __launch_bounds__(kPhaseThreads) k_dm_phase(DevMem mem, Map map, PhaseGeom g, Factor fac) {
     __shared__ double2 srow[32], scol[32];

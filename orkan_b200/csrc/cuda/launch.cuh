@@ -3,6 +3,8 @@
 // density-matrix phase-pass launcher used by gates and exp_diag.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "dm_direct.cuh"
 #include "dm_phase.cuh"
@@ -38,7 +40,7 @@ inline unsigned direct_grid(unsigned bits) { return grid_for(kDirectThreads, idx
 
 // Elementwise phase pass over a packed (layout 1) or tiled (layout 2) density matrix: one thread per element
 // up to kDirectSmall qubits (8 q: 4.0 against 6.2 us; from 11 q on the pass that skips whole inactive items
-// is faster, 8.3 against 12.4 us).
+// is faster, 8.3 against 12.4 us).  Above that, 1-qubit gates on packed storage go column by column.
 template <class Factor>
 int launch_phase(int layout, unsigned log_tile, void* rho, unsigned n, const Factor& fac, cudaStream_t st) {
     if (n <= kDirectSmall) {
@@ -47,6 +49,13 @@ int launch_phase(int layout, unsigned log_tile, void* rho, unsigned n, const Fac
         if (layout == 1) k_direct_phase<<<grid, kDirectThreads, 0, st>>>(mem, PackedMap{idx_t(1) << n}, n, fac);
         else k_direct_phase<<<grid, kDirectThreads, 0, st>>>(mem, TiledMap{idx_t(1) << n, log_tile}, n, fac);
         return finish_launch();
+    }
+    if constexpr (std::is_same<Factor, GateFactor1>::value) {
+        if (layout == 1 && n <= 21) {                   // (more blocks than a grid has beyond)
+            k_dm_phase_columns<<<(unsigned)phase_column_blocks(n), kColThreads, 0, st>>>(
+                DevMem{static_cast<double2*>(rho)}, PackedMap{idx_t(1) << n}, fac);
+            return finish_launch();
+        }
     }
     const PhaseGeom g = phase_geometry(n, layout == 2 ? log_tile : 5u);
     const unsigned grid = grid_for(phase_items_per_block(), g.items, kFullGrid);

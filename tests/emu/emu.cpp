@@ -168,6 +168,13 @@ unsigned emu_max_v() {
 
 template <class Factor>
 void run_phase(int layout, unsigned log_tile, const EmuMem& mem, unsigned n, const Factor& fac) {
+    if constexpr (std::is_same<Factor, GateFactor1>::value) {
+        if (layout == 1 && n > 10) {                    // as the GPU launcher picks it
+            for (idx_t b = 0; b < phase_column_blocks(n); ++b)
+                for (unsigned t = 0; t < kColThreads; ++t) dm_phase_columns(mem, PackedMap{idx_t(1) << n}, fac, b, t);
+            return;
+        }
+    }
     const PhaseGeom g = phase_geometry(n, layout == 2 ? log_tile : 5u);
     const unsigned grid = grid_for(1, g.items, kSms * 32u);
     for (unsigned b = 0; b < grid; ++b)
