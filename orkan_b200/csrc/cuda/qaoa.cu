@@ -615,7 +615,7 @@ int enqueue_kernels(const orkan_qaoa* b, const Plan& pl, cudaStream_t st) {
             P.C = L.C;
             P.kind = L.kind;
             P.status = b->d_out + b->count;
-            qaoa_pass_setup(P, L.n);
+            qaoa_pass_setup(P, L.n, L.bytes);
             rc = L.bytes ? launch_pass_t<uint8_t>(L.nt, L.grid, L.smem, P, T, st)
                          : launch_pass_t<double>(L.nt, L.grid, L.smem, P, T, st);
         } else {

@@ -302,8 +302,15 @@ struct QaoaPass {
     QaoaStage stage[kQaoaStageTable];
 };
 
-// Fill in the geometry and the stages of a pass of n-qubit instances.
-inline void qaoa_pass_setup(QaoaPass& P, unsigned n) {
+// Fill in the geometry and the stages of a pass of n-qubit instances, whose phases are read from the staged
+// tables (byte costs) or not.
+//
+// A stage that stores an item hands its buffers back before its arithmetic when a thread has one set, and the
+// next item's table may then arrive while slower threads still read this one's.  So where group 0 alone makes up
+// a middle pass (high items of 4 mixed bits, n = C + 4), byte costs take two stages: mixers A and the phase,
+// then mixers B and the stores.  (512 instances of 16 qubits, p = 4: 727 us.  A release after the stores instead
+// changes the registers of every byte-cost pass: 715 us there, but 16 instances of 24 qubits 5.71 against 5.59 ms.)
+inline void qaoa_pass_setup(QaoaPass& P, unsigned n, bool tables = true) {
     P.geo = qaoa_geo(n, P.C, P.kind);
     P.li = qaoa_log_items(n, P.C, P.kind);
     P.nreg = 0;
@@ -327,17 +334,23 @@ inline void qaoa_pass_setup(QaoaPass& P, unsigned n) {
     };
     if (!first)
         for (int g = m - 1; g > 0; --g) add(g, 0, -1);
-    add(0, first ? -1 : 0, last ? -1 : 1);
+    if (tables && !first && !last && m == 1 && qaoa_group_bits(P.geo, 0) == kQaoaGroup) {
+        add(0, 0, -1);
+        add(0, -1, 1);
+        P.stage[1].phase = -1;
+    } else {
+        add(0, first ? -1 : 0, last ? -1 : 1);
+    }
     if (!last)
         for (int g = 1; g < m; ++g) add(g, -1, 1);
     if (first) P.stage[0].src = kQaoaFromInit;
     P.stage[P.nreg - 1].dst = last ? kQaoaToMeasure : kQaoaToGlobal;
     // groups 0 and 1 of 16 amplitudes each stay within a half-warp, unless group 1 stores a
-    // high item (its sets are then numbered for the stores)
+    // high item (its sets are then numbered for the stores); the same group twice stays within a thread
     for (unsigned r = 0; r + 1 < P.nreg; ++r) {
         const QaoaStage &a = P.stage[r], &b = P.stage[r + 1];
         const bool pair = a.g + b.g == 1 && qaoa_group_bits(P.geo, 0) == 4 && qaoa_group_bits(P.geo, 1) == 4;
-        P.stage[r].warp_sync = pair && !(P.kind == kQaoaHigh && b.dst == kQaoaToGlobal);
+        P.stage[r].warp_sync = a.g == b.g || (pair && !(P.kind == kQaoaHigh && b.dst == kQaoaToGlobal));
     }
 }
 
@@ -492,7 +505,8 @@ ORKAN_HD double qaoa_m_stage(const QaoaGeo& g, const QaoaStage& sg, const QaoaIt
     const unsigned sets = 1u << (lc - K);
     const bool costs = sg.phase >= 0 || sg.dst == kQaoaToMeasure;
     const double gamma = J.gamma, fs = J.fs;
-    // J and the costs' place are read before the release: the next item overwrites J
+    // The release lets the next item overwrite J, the amplitudes and the phase table.  J and the costs' place are
+    // read before it; the table is not, so no stage reads the table and releases (qaoa_pass_setup).
     const double ka = J.ka, kb = J.kb;
     const int sa = J.sa, sb = J.sb;
     const idx_t item = J.item;
