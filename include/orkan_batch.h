@@ -69,6 +69,10 @@ int orkan_qaoa_cost_vector(orkan_qaoa_t *b, unsigned i, double *host_out);
 /* Waves, passes and kernel launches per orkan_qaoa_run. */
 int orkan_qaoa_stats(const orkan_qaoa_t *b, unsigned *waves, unsigned *launches);
 
+/* Test hook of the failure path: with on != 0 every wait of the passes for staged data runs out at
+ * once, and the launches return with their copies landed; 0 restores the default limit of 2^24 polls. */
+int orkan_qaoa_test_expire(orkan_qaoa_t *b, int on);
+
 void orkan_qaoa_destroy(orkan_qaoa_t *b);
 
 #ifdef __cplusplus

@@ -218,11 +218,11 @@ __global__ void __launch_bounds__(PassShape<C>::kBlock, 1)
         }
         if (!ok) *P.status = 1.0;
         asm volatile("cp.async.wait_all;\n" ::: "memory");
-        // the bulk copies land before the block's shared memory is given up: their items are
-        // computed first, except after an error
-        if (!ok)
+        // the bulk copies land before the block's shared memory is given up, also where a wait
+        // of the computing warps ran out and no one else sees to it
+        if (st == 0)
             for (unsigned b = 0; b < NB && b < k; ++b)
-                mb_wait(full + b, ((k - 1 - b) / NB) & 1u, P.wait_limit);
+                mb_wait(full + b, ((k - 1 - b) / NB) & 1u, kQaoaPolls);
         return;
     }
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kComputeRegs));
@@ -426,6 +426,7 @@ struct orkan_qaoa {
     size_t arena_bytes = 0, partial_cap = 0;
     QaoaInst* d_inst = nullptr;
     size_t inst_cap = 0;
+    unsigned long long polls = kQaoaPolls;  // limit of the passes' waits (orkan_qaoa_test_expire)
     // pinned host staging
     double* h_gamma = nullptr;
     QaoaRx* h_rx = nullptr;
@@ -616,6 +617,7 @@ int enqueue_kernels(const orkan_qaoa* b, const Plan& pl, cudaStream_t st) {
             P.kind = L.kind;
             P.status = b->d_out + b->count;
             qaoa_pass_setup(P, L.n, L.bytes);
+            P.wait_limit = b->polls;
             rc = L.bytes ? launch_pass_t<uint8_t>(L.nt, L.grid, L.smem, P, T, st)
                          : launch_pass_t<double>(L.nt, L.grid, L.smem, P, T, st);
         } else {
@@ -822,6 +824,12 @@ int orkan_qaoa_run(orkan_qaoa_t* b, const double* gammas, const double* betas, d
     if (b->h_out[b->count] != 0.0) return (int)cudaErrorLaunchTimeout;     // a wait for staged data ran out
     memcpy(means, b->h_out, (size_t)b->count * 8);
     return 0;
+}
+
+int orkan_qaoa_test_expire(orkan_qaoa_t* b, int on) {
+    if (!b) return (int)cudaErrorInvalidValue;
+    b->polls = on ? 0 : kQaoaPolls;
+    return rebuild(b);
 }
 
 int orkan_qaoa_config(const orkan_qaoa_t* b, unsigned n, unsigned* log_chunk, unsigned* threads, unsigned* ring) {

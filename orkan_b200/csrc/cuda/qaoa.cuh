@@ -280,6 +280,7 @@ struct QaoaStage {
 // A pass launch: its instances (all of one qubit count) and the pass's stages, computed once
 // on the host.
 constexpr unsigned kQaoaStageTable = 8;    // 2 m - 1 with m <= 4
+constexpr unsigned long long kQaoaPolls = 1ull << 24;   // limit of a bounded wait
 
 struct QaoaPass {
     const QaoaInst* inst;
@@ -315,7 +316,7 @@ inline void qaoa_pass_setup(QaoaPass& P, unsigned n, bool tables = true) {
     P.li = qaoa_log_items(n, P.C, P.kind);
     P.nreg = 0;
     P.layer_a = P.layer_b = P.layer_phase = -1;
-    P.wait_limit = 1ull << 24;
+    P.wait_limit = kQaoaPolls;
     for (auto& s : P.stage) s = QaoaStage{};
     if (P.kind == kQaoaFull) return;
     const int j = (int)P.pass, p = (int)P.p, m = (int)P.geo.m;
