@@ -672,6 +672,12 @@ int rebuild(orkan_qaoa* b) {
     return rc;
 }
 
+// The passes only ever set the status of their waits; whoever has read it set clears it.
+int clear_status(const orkan_qaoa* b, cudaStream_t st) {
+    const int rc = (int)cudaMemsetAsync(b->d_out + b->count, 0, 8, st);
+    return rc ? rc : (int)cudaStreamSynchronize(st);
+}
+
 // Angles into the pinned staging buffers; rx coefficients with the host's libm, as the
 // per-call rx takes them (cos(theta / 2), sin(theta / 2) with theta = 2 beta).
 void stage_angles(orkan_qaoa* b, const double* gammas, const double* betas) {
@@ -821,7 +827,10 @@ int orkan_qaoa_run(orkan_qaoa_t* b, const double* gammas, const double* betas, d
     stage_angles(b, gammas, betas);
     if ((rc = (int)cudaGraphLaunch(b->exec, st))) return rc;
     if ((rc = (int)cudaStreamSynchronize(st))) return rc;
-    if (b->h_out[b->count] != 0.0) return (int)cudaErrorLaunchTimeout;     // a wait for staged data ran out
+    if (b->h_out[b->count] != 0.0) {                        // a wait for staged data ran out
+        rc = clear_status(b, st);
+        return rc ? rc : (int)cudaErrorLaunchTimeout;
+    }
     memcpy(means, b->h_out, (size_t)b->count * 8);
     return 0;
 }
@@ -943,9 +952,11 @@ int orkan_qaoa_tune(orkan_qaoa_t* b, const double* gammas, const double* betas, 
                 if (ok) ok = cudaEventRecord(e1, b->cap) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess;
                 float ms = 0.f;
                 if (ok) ok = cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess;
-                if (!ok) {
+                double expired = 0.0;                       // a candidate whose waits ran out was not timed
+                if (ok) ok = cudaMemcpy(&expired, b->d_out + b->count, 8, cudaMemcpyDeviceToHost) == cudaSuccess;
+                if (!ok || expired != 0.0) {
                     cudaGetLastError();
-                    cudaStreamSynchronize(b->cap);
+                    clear_status(b, b->cap);
                     usable[ci] = false;
                     continue;
                 }
@@ -974,6 +985,7 @@ int orkan_qaoa_tune(orkan_qaoa_t* b, const double* gammas, const double* betas, 
             best = dflt_ms;
         }
         b->cfg[nq] = bestc;
+        if (best > 1e29f) continue;                         // nothing was timed: nothing to record
         char line[512];
         snprintf(line, sizeof line,
                  "{\"%s\": {\"C\": %u, \"threads\": %u, \"ring\": %u, \"ms_per_instance\": %.5f}}\n", key.c_str(),

@@ -49,3 +49,29 @@ def test_expired_waits_are_reported_and_leave_the_context_usable(f64_costs):
     fresh, g, b, want = make(f64_costs)
     with fresh:
         check(fresh, g, b, want)
+
+
+def test_the_next_run_of_the_batch_is_good_again():
+    bt, g, b, want = make(False)
+    with bt:
+        check(bt, g, b, want)
+        expire(bt, 1)
+        for _ in range(2):
+            with pytest.raises(OrkanError, match=str(TIMEOUT)):
+                bt.run(g, b)
+        expire(bt, 0)
+        check(bt, g, b, want)
+
+
+def test_tuning_takes_no_time_of_an_expired_candidate(tmp_path):
+    bt, g, b, want = make(False)
+    with bt:
+        before = {n: bt.config(n) for n in (9, 14, 16, 20)}
+        expire(bt, 1)
+        path = tmp_path / "tune.json"
+        bt.tune(g, b, str(path))
+        assert {n: bt.config(n) for n in before} == before          # the defaults: nothing was timed
+        recorded = path.read_text() if path.exists() else ""
+        assert "|n20|" not in recorded and "|n16|" not in recorded
+        expire(bt, 0)
+        check(bt, g, b, want)
