@@ -551,10 +551,17 @@ int fill_costs(orkan_qaoa* b, Graph& g, unsigned C) {
     return 0;
 }
 
+// The captured graph reads the buffers and the cost order of the plan that it was made for.
+void drop_exec(orkan_qaoa* b) {
+    if (b->exec) cudaGraphExecDestroy(b->exec);
+    b->exec = nullptr;
+}
+
 // Device side of a plan: the costs in the order of its passes, arena, partial sums, launch
 // shapes and the instance records.
 int upload_plan(orkan_qaoa* b, Plan& pl) {
     int rc;
+    drop_exec(b);
     bool filled = false;
     for (const auto& L : pl.launches) {
         if (L.what != 0) continue;
@@ -655,10 +662,6 @@ int rebuild(orkan_qaoa* b) {
     int rc = upload_plan(b, pl);
     if (rc) return rc;
     b->plan = pl;
-    if (b->exec) {
-        cudaGraphExecDestroy(b->exec);
-        b->exec = nullptr;
-    }
     cudaGraph_t g = nullptr;
     if ((rc = (int)cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal))) return rc;
     const int erc = enqueue_run(b, b->plan, b->cap);
@@ -668,6 +671,7 @@ int rebuild(orkan_qaoa* b) {
         return erc ? erc : rc;
     }
     rc = (int)cudaGraphInstantiate(&b->exec, g, 0);
+    if (rc) b->exec = nullptr;
     cudaGraphDestroy(g);
     return rc;
 }
@@ -824,6 +828,7 @@ int orkan_qaoa_run(orkan_qaoa_t* b, const double* gammas, const double* betas, d
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     int rc = (int)cudaStreamSynchronize(st);                // the staging buffers may still be read
     if (rc) return rc;
+    if (!b->exec && (rc = rebuild(b))) return rc;           // the last tuning ended in an error
     stage_angles(b, gammas, betas);
     if ((rc = (int)cudaGraphLaunch(b->exec, st))) return rc;
     if ((rc = (int)cudaStreamSynchronize(st))) return rc;
@@ -1005,7 +1010,7 @@ int orkan_qaoa_tune(orkan_qaoa_t* b, const double* gammas, const double* betas, 
 
 void orkan_qaoa_destroy(orkan_qaoa_t* b) {
     if (!b) return;
-    if (b->exec) cudaGraphExecDestroy(b->exec);
+    drop_exec(b);
     if (b->cap) cudaStreamDestroy(b->cap);
     cudaFree(b->d_costs);
     cudaFree(b->d_uv);
