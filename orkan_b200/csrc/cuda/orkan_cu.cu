@@ -126,11 +126,13 @@ int launch_direct(int layout, unsigned log_tile, void* rho, unsigned n, unsigned
     return finish_launch();
 }
 // Does an operation on 2 x 2 groups over bit q take the direct kernels?  All but the top qubit of large tiled
-// matrices do (14 q: 796 against 762 us there; 13 q 205 against 206), where every block's (r0, c1) tile is
-// transposed.  The engine's test hooks ask for an engine launch.
-bool direct_wins(int layout, unsigned n, unsigned q) {
+// matrices do, and, for operations that mix, the one below it: there every block's (r0, c1) tile is transposed.
+// Direct against engine, us, tiled: H on the top qubit 208 / 207 at 13 q, 796 / 762 at 14; one below 189 / 196,
+// 732 / 724 and 2886 / 2805 at 13, 14 and 15 q, where CX has 178 / 196, 685 / 723 and 2688 / 2817.  Packed is faster
+// direct throughout (15 q: H 3392 / 3727 on the top qubit).  The engine's test hooks ask for an engine launch.
+bool direct_wins(int layout, unsigned n, unsigned q, bool mixes) {
     if (g_engine_test_polls.load(std::memory_order_relaxed)) return false;
-    return layout == 1 || n < 14 || q + 1 < n;
+    return layout == 1 || n < 14 || q + (mixes ? 2u : 1u) < n;
 }
 // SWAP: one thread per element while the matrix lies in L2 (11 q: 16.5 against 22.7 us packed, 20.8 against 22.4
 // tiled; 12 q: 64 against 71, 99 against 66).
@@ -343,7 +345,7 @@ int orkan_cu_dm_unitary(int layout, unsigned log_tile, void* rho, unsigned n, un
     if (!rho || !qubits || !u || !layout_ok(layout, log_tile) || (k != 1 && k != 2) || n > 40)
         return (int)cudaErrorInvalidValue;
     if (!qubits_ok(n, k, qubits)) return (int)cudaErrorInvalidValue;
-    if (k == 1 && direct_wins(layout, n, qubits[0])) {
+    if (k == 1 && direct_wins(layout, n, qubits[0], true)) {
         DirectMix1 op;
         for (unsigned i = 0; i < 4; ++i) op.u[i] = ld_c(u, i);
         return launch_direct(layout, log_tile, rho, n, qubits[0], op, as_stream(stream));
@@ -373,7 +375,7 @@ int orkan_cu_dm_monomial(int layout, unsigned log_tile, void* rho, unsigned n, u
         op.phase[y] = ld_c(phase, y);
     }
     if (!qubits_ok(n, k, qubits)) return (int)cudaErrorInvalidValue;
-    if (n <= kDirectSwap && monomial_is_swap(op, k) && direct_wins(layout, n, 0)) {
+    if (n <= kDirectSwap && monomial_is_swap(op, k) && direct_wins(layout, n, 0, false)) {
         const DevMem mem{static_cast<double2*>(rho)};
         const unsigned grid = direct_grid(2 * n);
         if (layout == 1)
@@ -384,7 +386,7 @@ int orkan_cu_dm_monomial(int layout, unsigned log_tile, void* rho, unsigned n, u
                                                                           qubits[0], qubits[1]);
         return finish_launch();
     }
-    if (monomial_is_controlled_flip(op, k) && direct_wins(layout, n, qubits[k - 1])) {
+    if (monomial_is_controlled_flip(op, k) && direct_wins(layout, n, qubits[k - 1], false)) {
         unsigned long long ctrl = 0;
         for (unsigned j = 0; j + 1 < k; ++j) ctrl |= 1ull << qubits[j];
         const double2 p0 = op.phase[m - 2], p1 = op.phase[m - 1];
@@ -431,7 +433,7 @@ int orkan_cu_dm_phase(int layout, unsigned log_tile, void* rho, unsigned n, unsi
 int orkan_cu_dm_superop1(int layout, unsigned log_tile, void* rho, unsigned n, unsigned target, const double* sop,
                          void* stream) {
     if (!rho || !sop || !layout_ok(layout, log_tile) || target >= n || n > 40) return (int)cudaErrorInvalidValue;
-    if (direct_wins(layout, n, target)) {
+    if (direct_wins(layout, n, target, true)) {
         DirectSuper1 d;
         for (unsigned i = 0; i < 16; ++i) d.s[i] = ld_c(sop, i);
         return launch_direct(layout, log_tile, rho, n, target, d, as_stream(stream));
