@@ -25,8 +25,10 @@ def build() -> str:
     if not os.path.exists(LIB) or any(os.path.getmtime(d) > os.path.getmtime(LIB) for d in deps):
         import subprocess
         cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+        part = f"{LIB}.{os.getpid()}"                  # several test processes may build it at once
         subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I" + os.path.join(cuda, "include"),
-                        src, "-o", LIB], check=True)
+                        src, "-o", part], check=True)
+        os.replace(part, LIB)
     return LIB
 
 
