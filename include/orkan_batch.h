@@ -73,6 +73,10 @@ int orkan_qaoa_stats(const orkan_qaoa_t *b, unsigned *waves, unsigned *launches)
  * once, and the launches return with their copies landed; 0 restores the default limit of 2^24 polls. */
 int orkan_qaoa_test_expire(orkan_qaoa_t *b, int on);
 
+/* Test hook: from here on the batch's passes run in the form for builds whose compiler did not give
+ * them the registers that the default form divides among its warps. */
+int orkan_qaoa_test_plain_registers(orkan_qaoa_t *b);
+
 void orkan_qaoa_destroy(orkan_qaoa_t *b);
 
 #ifdef __cplusplus

@@ -138,7 +138,9 @@ __device__ __forceinline__ bool mb_wait(void* bar, unsigned parity, unsigned lon
 //
 // Registers: a block of 640 threads is launched with 96 each (61440); the staging warps give
 // back all but 32 (4096 in all) and the computing ones then take 112 (57344), which holds the
-// 16 amplitudes of a set (64) with little spilled.
+// 16 amplitudes of a set (64) with little spilled.  The split waits forever for registers that the launch
+// did not bring, so it is used where the compiler gave the kernel exactly those 96 (prepare_kernels);
+// SPLIT = false is the same pass at whatever it gave, for every other build.
 constexpr unsigned kStageThreads = 128;
 constexpr unsigned kComputeThreads = 512;
 constexpr unsigned kLaunchRegs = 96, kStageRegs = 32, kComputeRegs = 112;
@@ -165,7 +167,7 @@ struct PassShape {
 // 17.17, 22 qubits 1.41 against 4.13, 20 qubits 0.41 against 0.95, 16 qubits 0.086 against
 // 0.098; 8 weighted instances of 24 qubits at p = 6 5.89 against 19.8.  Half of the state's
 // amplitudes account for a factor of two, the staging and the shorter stages for the rest.
-template <class CostT, unsigned C>
+template <class CostT, unsigned C, bool SPLIT>
 __global__ void __launch_bounds__(PassShape<C>::kBlock, 1)
     k_qaoa_pass(const __grid_constant__ QaoaPass P, const QaoaTables T) {
     using Sh = PassShape<C>;
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(PassShape<C>::kBlock, 1)
     const unsigned warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const unsigned items = (unsigned)P.items;          // checked to fit by the host
     if (warp >= kComputeThreads / 32) {                // staging
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kStageRegs));
+        if constexpr (SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kStageRegs));
         const unsigned st = threadIdx.x - kComputeThreads;
         unsigned k = 0;
         bool ok = true;
@@ -225,7 +227,7 @@ __global__ void __launch_bounds__(PassShape<C>::kBlock, 1)
                 mb_wait(full + b, ((k - 1 - b) / NB) & 1u, kQaoaPolls);
         return;
     }
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kComputeRegs));
+    if constexpr (SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kComputeRegs));
     const unsigned gid = warp / (GT / 32), tid = threadIdx.x % GT;
     double* red = reinterpret_cast<double*>(smem_q + L.red) + gid * (GT / 32);
     auto group_sync = [&] { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + gid), "n"(GT) : "memory"); };
@@ -333,32 +335,49 @@ size_t pass_smem(unsigned kind, unsigned C, bool bytes, unsigned tstride) {
 }
 
 template <class K>
-int allow_smem(K kern, int regs = 0) {
-    if (regs) {                                        // the register split counts on the launch's registers
-        cudaFuncAttributes fa;
-        const int rc = (int)cudaFuncGetAttributes(&fa, kern);
-        if (rc) return rc;
-        if (fa.numRegs != regs) return (int)cudaErrorInvalidConfiguration;
-    }
+int allow_smem(K kern) {
     return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
 }
-// Sets the kernels' shared-memory limits on the current device (before any graph capture).
-int prepare_kernels() {
+// *split is cleared unless the kernel was compiled to the registers of the split.
+template <class CostT, unsigned C>
+int prepare_pass(bool* split) {
+    cudaFuncAttributes fa;
+    const int rc = (int)cudaFuncGetAttributes(&fa, k_qaoa_pass<CostT, C, true>);
+    if (!rc && fa.numRegs != (int)kLaunchRegs) *split = false;
+    return rc ? rc : allow_smem(k_qaoa_pass<CostT, C, true>);
+}
+int prepare_plain() {
     int rc;
-    if ((rc = allow_smem(k_qaoa_pass<uint8_t, 11>, kLaunchRegs)) || (rc = allow_smem(k_qaoa_pass<uint8_t, 12>, kLaunchRegs)) ||
-        (rc = allow_smem(k_qaoa_pass<uint8_t, 13>, kLaunchRegs)) || (rc = allow_smem(k_qaoa_pass<double, 11>, kLaunchRegs)) ||
-        (rc = allow_smem(k_qaoa_pass<double, 12>, kLaunchRegs)) || (rc = allow_smem(k_qaoa_pass<double, 13>, kLaunchRegs)) ||
-        (rc = allow_smem(k_qaoa_full<uint8_t>)) || (rc = allow_smem(k_qaoa_full<double>)))
+    if ((rc = allow_smem(k_qaoa_pass<uint8_t, 11, false>)) || (rc = allow_smem(k_qaoa_pass<uint8_t, 12, false>)) ||
+        (rc = allow_smem(k_qaoa_pass<uint8_t, 13, false>)) || (rc = allow_smem(k_qaoa_pass<double, 11, false>)) ||
+        (rc = allow_smem(k_qaoa_pass<double, 12, false>)) || (rc = allow_smem(k_qaoa_pass<double, 13, false>)))
         return rc;
     return 0;
 }
+// Sets the kernels' shared-memory limits on the current device (before any graph capture) and picks the form.
+int prepare_kernels(bool* split) {
+    *split = true;
+    int rc;
+    if ((rc = prepare_pass<uint8_t, 11>(split)) || (rc = prepare_pass<uint8_t, 12>(split)) ||
+        (rc = prepare_pass<uint8_t, 13>(split)) || (rc = prepare_pass<double, 11>(split)) ||
+        (rc = prepare_pass<double, 12>(split)) || (rc = prepare_pass<double, 13>(split)) ||
+        (rc = allow_smem(k_qaoa_full<uint8_t>)) || (rc = allow_smem(k_qaoa_full<double>)))
+        return rc;
+    return *split ? 0 : prepare_plain();
+}
 
+template <class CostT, unsigned C>
+void launch_chunks(bool split, unsigned grid, size_t smem, const QaoaPass& P, const QaoaTables& T, cudaStream_t st) {
+    if (split) k_qaoa_pass<CostT, C, true><<<grid, PassShape<C>::kBlock, smem, st>>>(P, T);
+    else k_qaoa_pass<CostT, C, false><<<grid, PassShape<C>::kBlock, smem, st>>>(P, T);
+}
 template <class CostT>
-int launch_pass_t(unsigned nt, unsigned grid, size_t smem, const QaoaPass& P, const QaoaTables& T, cudaStream_t st) {
+int launch_pass_t(bool split, unsigned nt, unsigned grid, size_t smem, const QaoaPass& P, const QaoaTables& T,
+                  cudaStream_t st) {
     if (P.kind == kQaoaFull) k_qaoa_full<CostT><<<grid, nt, smem, st>>>(P, T);
-    else if (P.C == 11) k_qaoa_pass<CostT, 11><<<grid, PassShape<11>::kBlock, smem, st>>>(P, T);
-    else if (P.C == 12) k_qaoa_pass<CostT, 12><<<grid, PassShape<12>::kBlock, smem, st>>>(P, T);
-    else k_qaoa_pass<CostT, 13><<<grid, PassShape<13>::kBlock, smem, st>>>(P, T);
+    else if (P.C == 11) launch_chunks<CostT, 11>(split, grid, smem, P, T, st);
+    else if (P.C == 12) launch_chunks<CostT, 12>(split, grid, smem, P, T, st);
+    else launch_chunks<CostT, 13>(split, grid, smem, P, T, st);
     return (int)cudaGetLastError();
 }
 
@@ -426,6 +445,7 @@ struct orkan_qaoa {
     size_t arena_bytes = 0, partial_cap = 0;
     QaoaInst* d_inst = nullptr;
     size_t inst_cap = 0;
+    bool split = true;                      // the passes re-divide their registers
     unsigned long long polls = kQaoaPolls;  // limit of the passes' waits (orkan_qaoa_test_expire)
     // pinned host staging
     double* h_gamma = nullptr;
@@ -625,8 +645,8 @@ int enqueue_kernels(const orkan_qaoa* b, const Plan& pl, cudaStream_t st) {
             P.status = b->d_out + b->count;
             qaoa_pass_setup(P, L.n, L.bytes);
             P.wait_limit = b->polls;
-            rc = L.bytes ? launch_pass_t<uint8_t>(L.nt, L.grid, L.smem, P, T, st)
-                         : launch_pass_t<double>(L.nt, L.grid, L.smem, P, T, st);
+            rc = L.bytes ? launch_pass_t<uint8_t>(b->split, L.nt, L.grid, L.smem, P, T, st)
+                         : launch_pass_t<double>(b->split, L.nt, L.grid, L.smem, P, T, st);
         } else {
             k_qaoa_fold<<<L.ninst, kFoldThreads, 0, st>>>(inst, L.ninst, b->d_partial + L.partial_off, L.items, b->d_rx,
                                                           b->p, b->d_out);
@@ -807,7 +827,7 @@ int orkan_qaoa_create(orkan_qaoa_t** out, unsigned count, const unsigned* n_qubi
         (rc = dalloc(&b->d_table, b->any_bytes ? np * b->tstride : 1)) || (rc = dalloc(&b->d_out, (size_t)count + 1)) ||
         (rc = (int)cudaMallocHost(&b->h_gamma, np * 8)) || (rc = (int)cudaMallocHost(&b->h_rx, np * sizeof(QaoaRx))) ||
         (rc = (int)cudaMallocHost(&b->h_out, ((size_t)count + 1) * 8)) ||
-        (rc = (int)cudaMemset(b->d_out, 0, ((size_t)count + 1) * 8)) || (rc = prepare_kernels()) ||
+        (rc = (int)cudaMemset(b->d_out, 0, ((size_t)count + 1) * 8)) || (rc = prepare_kernels(&b->split)) ||
         (rc = (int)cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking))) {
         orkan_qaoa_destroy(b);
         return rc;
@@ -844,6 +864,13 @@ int orkan_qaoa_test_expire(orkan_qaoa_t* b, int on) {
     if (!b) return (int)cudaErrorInvalidValue;
     b->polls = on ? 0 : kQaoaPolls;
     return rebuild(b);
+}
+
+int orkan_qaoa_test_plain_registers(orkan_qaoa_t* b) {
+    if (!b) return (int)cudaErrorInvalidValue;
+    b->split = false;
+    const int rc = prepare_plain();
+    return rc ? rc : rebuild(b);
 }
 
 int orkan_qaoa_config(const orkan_qaoa_t* b, unsigned n, unsigned* log_chunk, unsigned* threads, unsigned* ring) {
