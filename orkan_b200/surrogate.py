@@ -185,24 +185,39 @@ class NoisyEvaluator:
     """Exact FP64 <C> of the noisy circuit on a density matrix through the per-call API:
     |+><+|, then per layer exp_diag(cost, gamma_k) and, on every qubit, rx(2 beta_k) followed by a
     depolarizing channel -- applied as one channel_1q_layer with the superoperator of the Kraus
-    set {K_i Rx} on every qubit -- then mean(cost).  The costs stay on the device, and a state is
-    kept for the next evaluation (one per thread that evaluates at a time, at most four)."""
+    set {K_i Rx} on every qubit -- then mean(cost).  `cost` may be changed between calls: a call
+    copies it to the device where its values are new.  A state is kept for the next evaluation (one per thread that
+    evaluates at a time, at most four)."""
 
     def __init__(self, ork, n, edges, weights, p, prob, kind="tiled"):
-        import torch
         self.ork, self.n, self.p, self.prob, self.kind = ork, n, p, prob, kind
         x = np.arange(1 << n, dtype=np.int64)
         cost = np.zeros(1 << n)
         for e, (u, v) in enumerate(edges):
             cost += (1.0 if weights is None else float(weights[e])) * (((x >> u) ^ (x >> v)) & 1)
         self.cost = cost
-        self._cost = torch.from_numpy(cost).cuda()
         self.kraus = depolarizing_kraus(prob)
         self.evals = 0
+        self._staged = None
         self._states = []
 
     def one(self, g, b):
         return self._run(np.asarray(g)[None], np.asarray(b)[None])[0]
+
+    def _device_cost(self):
+        """(pointer, what keeps it alive) of the costs as they are now: the copy of an earlier call
+        serves where the values are the same."""
+        if isinstance(self.cost, int):                     # a device pointer, as exp_diag and mean take it
+            return self.cost, None
+        import torch
+        now = np.asarray(self.cost, dtype=np.float64).reshape(-1)
+        if now.size < 1 << self.n:
+            raise OrkanError("cost has fewer than 2^n entries")
+        device, staged = torch.cuda.current_device(), self._staged
+        if staged is None or staged[0] != device or not np.array_equal(staged[1], now):
+            host = now.copy()
+            staged = self._staged = (device, host, torch.from_numpy(host).cuda())
+        return int(staged[2].data_ptr()), staged[2]
 
     def _run(self, gs, bs):
         ork, n = self.ork, self.n
@@ -212,7 +227,8 @@ class NoisyEvaluator:
         rx[..., 0, 1] = rx[..., 1, 0] = -1j * np.sin(half)
         sops = sum(np.einsum("...ik,...jl->...ijkl", k @ rx, np.conj(k @ rx)) for k in self.kraus)
         sops = sops.reshape(half.shape + (4, 4))
-        cost, qubits = int(self._cost.data_ptr()), np.arange(n, dtype=np.uint8)
+        qubits = np.arange(n, dtype=np.uint8)
+        cost, keep = self._device_cost()
         try:
             st = self._states.pop()
         except IndexError:
