@@ -177,17 +177,22 @@ def depolarizing_kraus(prob):
 
 
 def rx_matrix(theta):
-    c, s = np.cos(theta / 2.0), np.sin(theta / 2.0)
-    return np.array([[c, -1j * s], [-1j * s, c]])
+    """rx(theta), 2 x 2; for an array of angles one matrix each in the last two axes."""
+    half = np.asarray(theta) / 2.0
+    m = np.empty(half.shape + (2, 2), dtype=np.complex128)
+    m[..., 0, 0] = m[..., 1, 1] = np.cos(half)
+    m[..., 0, 1] = m[..., 1, 0] = -1j * np.sin(half)
+    return m
 
 
 class NoisyEvaluator:
     """Exact FP64 <C> of the noisy circuit on a density matrix through the per-call API:
     |+><+|, then per layer exp_diag(cost, gamma_k) and, on every qubit, rx(2 beta_k) followed by a
     depolarizing channel -- applied as one channel_1q_layer with the superoperator of the Kraus
-    set {K_i Rx} on every qubit -- then mean(cost).  `cost` may be changed between calls: a call
-    copies it to the device where its values are new.  A state is kept for the next evaluation (one per thread that
-    evaluates at a time, at most four)."""
+    set {K_i Rx} on every qubit -- then mean(cost).  Attributes may be changed between
+    calls; a call copies `cost` to the device where its values are new.  A state (138 MB at 12
+    qubits) is kept for the next evaluation, one per thread that evaluates at a time, at most four;
+    close() frees them."""
 
     def __init__(self, ork, n, edges, weights, p, prob, kind="tiled"):
         self.ork, self.n, self.p, self.prob, self.kind = ork, n, p, prob, kind
@@ -202,9 +207,9 @@ class NoisyEvaluator:
         self._states = []
 
     def one(self, g, b):
-        return self._run(np.asarray(g)[None], np.asarray(b)[None])[0]
+        return float(self._run(np.asarray(g)[None], np.asarray(b)[None])[0])
 
-    def _device_cost(self):
+    def _device_cost(self, device):
         """(pointer, what keeps it alive) of the costs as they are now: the copy of an earlier call
         serves where the values are the same."""
         if isinstance(self.cost, int):                     # a device pointer, as exp_diag and mean take it
@@ -213,29 +218,39 @@ class NoisyEvaluator:
         now = np.asarray(self.cost, dtype=np.float64).reshape(-1)
         if now.size < 1 << self.n:
             raise OrkanError("cost has fewer than 2^n entries")
-        device, staged = torch.cuda.current_device(), self._staged
+        staged = self._staged
         if staged is None or staged[0] != device or not np.array_equal(staged[1], now):
             host = now.copy()
             staged = self._staged = (device, host, torch.from_numpy(host).cuda())
         return int(staged[2].data_ptr()), staged[2]
 
+    def _state(self, device):
+        """(key, state): a kept state of this device, layout and qubit count, or a new one."""
+        key = (device, self.kind, self.n)
+        while self._states:
+            try:
+                kept = self._states.pop()
+            except IndexError:                             # another thread took the last one
+                break
+            if kept[0] == key:
+                return kept
+            self.ork.free(kept[1])
+        return key, self.ork.state(self.kind, self.n)
+
     def _run(self, gs, bs):
-        ork, n = self.ork, self.n
+        import torch
+        ork, n, count = self.ork, self.n, min(len(gs), len(bs))
         half = np.asarray(bs, dtype=np.float64)
-        rx = np.empty(half.shape + (2, 2), dtype=np.complex128)
-        rx[..., 0, 0] = rx[..., 1, 1] = np.cos(half)
-        rx[..., 0, 1] = rx[..., 1, 0] = -1j * np.sin(half)
+        rx = rx_matrix(2.0 * half)
         sops = sum(np.einsum("...ik,...jl->...ijkl", k @ rx, np.conj(k @ rx)) for k in self.kraus)
         sops = sops.reshape(half.shape + (4, 4))
         qubits = np.arange(n, dtype=np.uint8)
-        cost, keep = self._device_cost()
+        out = np.empty(count)
+        device = torch.cuda.current_device()
+        cost, keep = self._device_cost(device)
+        key, st = self._state(device)
         try:
-            st = self._states.pop()
-        except IndexError:
-            st = ork.state(self.kind, n)
-        out = np.empty(len(gs))
-        try:
-            for e, g in enumerate(gs):
+            for e, g in enumerate(gs[:count]):
                 rc = ork.lib.orkan_cu_fill(st.type, ork.log_tile, st.data, n, 1.0 / (1 << n), 0.0,
                                            ork.lib.orkan_get_stream())
                 if rc:
@@ -244,12 +259,15 @@ class NoisyEvaluator:
                     ork.exp_diag(st, cost, float(g[k]))
                     ork.channel_1q_layer(st, sops[e, k], qubits)
                 out[e] = ork.mean(st, cost)
-        finally:
-            if len(self._states) < 4:
-                self._states.append(st)
-            else:
-                ork.free(st)
-        self.evals += len(gs)
+        except BaseException:
+            ork.sync()                                     # launches may still use the state and the costs
+            ork.free(st)
+            raise
+        if len(self._states) < 4:
+            self._states.append((key, st))
+        else:
+            ork.free(st)
+        self.evals += count
         return out
 
     def __call__(self, gammas, betas):
@@ -257,7 +275,7 @@ class NoisyEvaluator:
 
     def close(self):
         while self._states:
-            self.ork.free(self._states.pop())
+            self.ork.free(self._states.pop()[1])
 
     def __del__(self):
         try:

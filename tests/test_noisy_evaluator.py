@@ -44,3 +44,32 @@ def test_costs_changed_in_place_and_replaced(ork5):
     ev.cost = [float(x % 7) for x in range(32)]            # a list, as exp_diag and mean take one
     assert np.abs(ev(g, b) - oracle("tiled", 5, np.array(ev.cost), g, b)).max() < TOL
     assert abs(ev.one(g[1], b[1]) - ev(g, b)[1]) < TOL
+
+
+@pytest.mark.gpu
+def test_layout_and_qubit_count_changed_between_calls(ork5):
+    ev = NoisyEvaluator(ork5, 5, EDGES, WEIGHTS, 2, PROB)
+    g, b = angles(2, 2)
+    ev(g, b)
+    ev.kind = "packed"
+    assert np.abs(ev(g, b) - oracle("packed", 5, ev.cost, g, b)).max() < TOL
+    ev.n, ev.cost = 7, R.maxcut_cost(7, EDGES + [(5, 6), (0, 6)])
+    assert np.abs(ev(g, b) - oracle("packed", 7, ev.cost, g, b)).max() < TOL
+    ev.close()
+    assert np.abs(ev(g, b) - oracle("packed", 7, ev.cost, g, b)).max() < TOL
+
+
+@pytest.mark.gpu
+def test_angle_sets_are_paired_and_a_failed_call_keeps_no_state(ork5):
+    ev = NoisyEvaluator(ork5, 5, EDGES, WEIGHTS, 2, PROB)
+    g, b = angles(3, 2)
+    want = oracle("tiled", 5, ev.cost, g, b)
+    assert np.abs(ev(g, b[:2]) - want[:2]).max() < TOL     # as zip(gammas, betas)
+    assert np.abs(ev(g[:1], b) - want[:1]).max() < TOL
+    assert type(ev.one(g[2], b[2])) is float
+    assert len(ev(g[:0], b[:0])) == 0
+    with pytest.raises(IndexError):
+        ev(g[:, :1], b)                                    # too few angles for two layers
+    assert np.abs(ev(g, b) - want).max() < TOL
+    ev.close()
+    assert not ev._states
