@@ -189,8 +189,13 @@ class Orkan:
 
     # ---- operations --------------------------------------------------------------
     def gate(self, s: StateT, name: str, qubits, theta: float | None = None) -> None:
-        fn = self._gates.get(name) or getattr(self.lib, name)
-        try:                                   # plain ints and floats need no conversion here
+        if qubits.__class__ is not tuple:
+            qubits = tuple(qubits)             # an iterator is read once
+        try:
+            fn = self._gates[name]
+        except KeyError:
+            fn = getattr(self.lib, name)
+        try:                                   # integers and floats need no conversion here
             if theta is None:
                 fn(s, *qubits)
             else:
