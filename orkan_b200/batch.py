@@ -217,14 +217,24 @@ def erdos_renyi_graph(n: int, prob: float, rng) -> list[tuple[int, int]]:
     return [(u, v) for u in range(n) for v in range(u + 1, n) if rng.random() < prob]
 
 
+def ignored_settings(config, chunk=0, threads=None, ring=None) -> str:
+    """What was asked for and is not the configuration (log2 chunk, threads, ring) in use."""
+    wrong = [f"{name} {asked} (in use: {used})"
+             for name, asked, used in (("chunk", chunk or None, config[0]), ("threads", threads, config[1]),
+                                       ("ring", ring, config[2])) if asked is not None and asked != used]
+    return "not used: " + ", ".join(wrong) if wrong else ""
+
+
 def _main(argv=None):
     """Run one batch of 3-regular MaxCut instances: python -m orkan_b200.batch --count 64
-    --qubits 20 [--p 4 --chunk 12 --threads 256 --ring 1 --runs 2].  With --chunk the
-    launch configuration of that qubit count is set through a tuner cache file instead of
-    tuning.  Prints the configuration, the first mean and the time per run."""
+    --qubits 20 [--p 4 --chunk 12 --runs 2].  With --chunk the launch configuration of that
+    qubit count is set through a tuner cache file instead of tuning.  The chunk alone decides
+    threads and ring; --threads and --ring are still taken, and a note says so where they ask
+    for others.  Prints the configuration, the first mean and the time per run."""
     import argparse
     import json
     import os
+    import sys
     import tempfile
     import time
 
@@ -235,8 +245,8 @@ def _main(argv=None):
     ap.add_argument("--qubits", type=int, default=20)
     ap.add_argument("--p", type=int, default=4)
     ap.add_argument("--chunk", type=int, default=0)
-    ap.add_argument("--threads", type=int, default=256)
-    ap.add_argument("--ring", type=int, default=1)
+    ap.add_argument("--threads", type=int, default=None)
+    ap.add_argument("--ring", type=int, default=None)
     ap.add_argument("--runs", type=int, default=2)
     ap.add_argument("--f64", action="store_true")
     a = ap.parse_args(argv)
@@ -251,9 +261,12 @@ def _main(argv=None):
         key = f"{torch.cuda.get_device_name()}|n{a.qubits}|p{a.p}|{'f64' if a.f64 else 'u8'}|v3"
         fd, path = tempfile.mkstemp(suffix=".json")
         with os.fdopen(fd, "w") as f:
-            f.write(json.dumps({key: {"C": a.chunk, "threads": a.threads, "ring": a.ring}}) + "\n")
+            f.write(json.dumps({key: {"C": a.chunk, "threads": a.threads or 256, "ring": a.ring or 1}}) + "\n")
         bt.tune(g, b, path)
         os.unlink(path)
+    note = ignored_settings(bt.config(a.qubits), a.chunk, a.threads, a.ring)
+    if note:
+        print(note, file=sys.stderr)
     means = bt.run(g, b)
     t0 = time.perf_counter()
     for _ in range(a.runs):
