@@ -280,6 +280,7 @@ struct QaoaStage {
 // A pass launch: its instances (all of one qubit count) and the pass's stages, computed once
 // on the host.
 constexpr unsigned kQaoaStageTable = 8;    // 2 m - 1 with m <= 4
+static_assert((kQaoaMaxC + kQaoaGroup - 1) / kQaoaGroup <= (kQaoaStageTable + 1) / 2, "the stages of every pass fit");
 constexpr unsigned long long kQaoaPolls = 1ull << 24;   // limit of a bounded wait
 
 struct QaoaPass {
@@ -319,7 +320,8 @@ inline void qaoa_pass_setup(QaoaPass& P, unsigned n, bool tables = true) {
     P.wait_limit = kQaoaPolls;
     for (auto& s : P.stage) s = QaoaStage{};
     if (P.kind == kQaoaFull) return;
-    const int j = (int)P.pass, p = (int)P.p, m = (int)P.geo.m;
+    const int j = (int)P.pass, p = (int)P.p, most = (kQaoaStageTable + 1) / 2;
+    const int m = (int)P.geo.m < most ? (int)P.geo.m : most;       // (kQaoaMaxC bits are 4 groups)
     const bool first = j == 0, last = j == p;
     P.layer_a = first ? -1 : j - 1;
     P.layer_b = last ? -1 : j;
