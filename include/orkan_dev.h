@@ -61,7 +61,8 @@ void channel_2q(state_t *state, const superop_t *sop, qubit_t q0, qubit_t q1);
 
 /* count 1-qubit channels on a density matrix, sops[i] on targets[i], in the given order: the same
  * map as count calls of channel_1q, in fewer passes over the matrix (channels on different
- * qubits commute; up to six qubits share a pass).  Validation as channel_1q.  No counterpart in
+ * qubits commute; up to six qubits share a pass).  The superoperators map Hermitian matrices to
+ * Hermitian ones, as those of every Kraus set do.  Validation as channel_1q.  No counterpart in
  * the reference, which applies every channel as its own pass (src/channel/channel.c:52-85). */
 void channel_1q_layer(state_t *state, const superop_t *sops, const qubit_t *targets, unsigned count);
 

@@ -45,11 +45,12 @@ ORKAN_HD void direct_pair(idx_t t, unsigned b, idx_t* row, idx_t* col) {
     *col = Map::kRowContig ? slow : fast;
 }
 
-// Operations on a group x = (x00, x01, x10, x11).
+// Operations on a group x = (x00, x01, x10, x11).  above: (r0, c1) lies above the diagonal, and its conjugate
+// (c1, r0) is what is stored.
 struct DirectMix1 {
     double2 u[4];
     ORKAN_HD bool active(idx_t, idx_t) const { return true; }
-    ORKAN_HD void apply(const double2 (&x)[4], double2 (&z)[4], idx_t, idx_t) const {
+    ORKAN_HD void apply(const double2 (&x)[4], double2 (&z)[4], idx_t, idx_t, bool) const {
         double2 y[4];                                  // y = u x, z = y u^dagger
         for (unsigned j = 0; j < 2; ++j) {
             y[j] = cadd(cmul(u[0], x[j]), cmul(u[1], x[2 + j]));
@@ -64,12 +65,19 @@ struct DirectMix1 {
 struct DirectSuper1 {
     double2 s[16];
     ORKAN_HD bool active(idx_t, idx_t) const { return true; }
-    ORKAN_HD void apply(const double2 (&x)[4], double2 (&z)[4], idx_t, idx_t) const {
+    // A superoperator that does not map Hermitian matrices to Hermitian ones has two values for (r0, c1): row 01 of its
+    // own, and the conjugate of what row 10 gives (c1, r0).  The stored element's counts.
+    ORKAN_HD void apply(const double2 (&x)[4], double2 (&z)[4], idx_t, idx_t, bool above) const {
 #pragma unroll
         for (unsigned m = 0; m < 4; ++m) {
             double2 acc = c2(0.0, 0.0);
+            if (m == 1 && above) {
 #pragma unroll
-            for (unsigned j = 0; j < 4; ++j) super_fma(acc, s[4 * m + j], x[j]);
+                for (unsigned j = 0; j < 4; ++j) super_fma(acc, cconj(s[8 + (j == 1 ? 2 : j == 2 ? 1 : j)]), x[j]);
+            } else {
+#pragma unroll
+                for (unsigned j = 0; j < 4; ++j) super_fma(acc, s[4 * m + j], x[j]);
+            }
             z[m] = acc;
         }
     }
@@ -82,7 +90,7 @@ struct DirectFlip {
     unsigned long long ctrl;
     double2 p0, p1;
     ORKAN_HD bool active(idx_t r0, idx_t c0) const { return (r0 & ctrl) == ctrl || (c0 & ctrl) == ctrl; }
-    ORKAN_HD void apply(const double2 (&x)[4], double2 (&z)[4], idx_t r0, idx_t c0) const {
+    ORKAN_HD void apply(const double2 (&x)[4], double2 (&z)[4], idx_t r0, idx_t c0, bool) const {
         const bool cr = (r0 & ctrl) == ctrl, cc = (c0 & ctrl) == ctrl;
         double2 y[4];
 #pragma unroll
@@ -119,7 +127,7 @@ ORKAN_HD void direct_group(const Mem& mem, const Map& map, unsigned q, const Op&
     x[2] = mem.ld(map.at(r1, c0));
     x[3] = mem.ld(map.at(r1, c1));
     x[1] = u == v ? cconj(x[2]) : below ? mem.ld(map.at(r0, c1)) : cconj(mem.ld(map.at(c1, r0)));
-    op.apply(x, z, r0, c0);
+    op.apply(x, z, r0, c0, !below);
     direct_store(mem, map, r0, c0, z[0]);
     direct_store(mem, map, r1, c0, z[2]);
     direct_store(mem, map, r1, c1, z[3]);
@@ -169,61 +177,70 @@ ORKAN_HD void direct_tile_uv(const DirectWhere& w, unsigned f, unsigned o, idx_t
     *u = w.U * kDirectTile + (Map::kRowContig ? f : o);
     *v = w.V * kDirectTile + (Map::kRowContig ? o : f);
 }
-template <class Map, class Mem, class Op>
-ORKAN_HD void direct_tile_phase(int phase, const Mem& mem, const Map& map, unsigned q, const Op& op,
-                                const DirectWhere& w, double2* sh, unsigned tid, unsigned nthr) {
-    constexpr unsigned N = kDirectTile * kDirectTile;
+// Can an element off the diagonal tiles have a mirror image?  (Storage tiles of 32 and less hold no two rows of
+// a tile of groups there.)
+template <class Map>
+ORKAN_HD bool direct_mirrors(const Map& map) { return Map::kMirrors && map.log_tdim() > 5; }
+
+// Phase 1: the update of a tile's groups.  TR: the tile of (c1, r0) is staged in sh.
+template <bool TR, class Map, class Mem, class Op>
+ORKAN_HD void direct_tile_update(const Mem& mem, const Map& map, unsigned q, const Op& op, const DirectWhere& w,
+                                 double2* sh, unsigned tid, unsigned nthr) {
     const idx_t bit = idx_t(1) << q;
-    const bool mirrors = Map::kMirrors && map.log_tdim() > 5;      // smaller tiles hold no two rows of a tile here
-    auto put = [&](idx_t r, idx_t c, double2 x) {
-        if (mirrors) direct_store(mem, map, r, c, x);
-        else mem.st(map.at(r, c), x);
-    };
-    if (phase != 1) {
-        for (unsigned e = tid; e < N; e += nthr) {
-            const unsigned o = e % kDirectTile, f = e / kDirectTile;
-            idx_t u, v;
-            direct_tile_uv<Map>(w, f, o, &u, &v);
-            const idx_t r0 = insert0(u, q), c0 = insert0(v, q), c1 = c0 | bit;
-            if (!op.active(r0, c0)) continue;
-            double2& s = sh[f * kDirectPitch + o];
-            if (phase == 0) s = cconj(mem.ld(map.at(c1, r0)));
-            else put(c1, r0, cconj(s));
-        }
-        return;
-    }
+    const bool mirrors = direct_mirrors(map);
     // one group at a time: two (their loads issued together) need 78-128 registers instead of 56-80, and
     // the blocks lost cost more than they gain (H at 14 q: 740 against 640 us tiled, 650 against 645 packed)
 #ifdef __CUDA_ARCH__
 #pragma unroll 1
 #endif
-    for (unsigned e = tid; e < N; e += nthr) {
+    for (unsigned e = tid; e < kDirectTile * kDirectTile; e += nthr) {
         const unsigned f = e % kDirectTile, o = e / kDirectTile;
         idx_t u, v;
         direct_tile_uv<Map>(w, f, o, &u, &v);
         const idx_t r0 = insert0(u, q), c0 = insert0(v, q), r1 = r0 | bit, c1 = c0 | bit;
         if (!op.active(r0, c0)) continue;
         const idx_t a00 = map.at(r0, c0), a10 = map.at(r1, c0), a11 = map.at(r1, c1);
-        const idx_t a01 = w.transposed ? 0 : map.at(r0, c1);
+        const idx_t a01 = TR ? 0 : map.at(r0, c1);
         double2& s01 = sh[f * kDirectPitch + o];
         double2 x[4], z[4];
         x[0] = mem.ld(a00);
         x[2] = mem.ld(a10);
         x[3] = mem.ld(a11);
-        x[1] = w.transposed ? s01 : mem.ld(a01);
-        op.apply(x, z, r0, c0);
+        x[1] = TR ? s01 : mem.ld(a01);
+        op.apply(x, z, r0, c0, TR);
         if (mirrors) {
-            put(r0, c0, z[0]);
-            put(r1, c0, z[2]);
-            put(r1, c1, z[3]);
+            direct_store(mem, map, r0, c0, z[0]);
+            direct_store(mem, map, r1, c0, z[2]);
+            direct_store(mem, map, r1, c1, z[3]);
         } else {
             mem.st(a00, z[0]);
             mem.st(a10, z[2]);
             mem.st(a11, z[3]);
         }
-        if (w.transposed) s01 = z[1];
-        else if (mirrors) put(r0, c1, z[1]);
+        if (TR) s01 = z[1];
+        else if (mirrors) direct_store(mem, map, r0, c1, z[1]);
         else mem.st(a01, z[1]);
+    }
+}
+template <class Map, class Mem, class Op>
+ORKAN_HD void direct_tile_phase(int phase, const Mem& mem, const Map& map, unsigned q, const Op& op,
+                                const DirectWhere& w, double2* sh, unsigned tid, unsigned nthr) {
+    if (phase == 1) {
+        if (w.transposed) direct_tile_update<true>(mem, map, q, op, w, sh, tid, nthr);
+        else direct_tile_update<false>(mem, map, q, op, w, sh, tid, nthr);
+        return;
+    }
+    const idx_t bit = idx_t(1) << q;
+    for (unsigned e = tid; e < kDirectTile * kDirectTile; e += nthr) {
+        const unsigned o = e % kDirectTile, f = e / kDirectTile;
+        idx_t u, v;
+        direct_tile_uv<Map>(w, f, o, &u, &v);
+        const idx_t r0 = insert0(u, q), c0 = insert0(v, q), c1 = c0 | bit;
+        if (!op.active(r0, c0)) continue;
+        double2& s = sh[f * kDirectPitch + o];
+        if (phase == 0) s = cconj(mem.ld(map.at(c1, r0)));
+        else if (direct_mirrors(map)) direct_store(mem, map, c1, r0, cconj(s));
+        else mem.st(map.at(c1, r0), cconj(s));
     }
 }
 
