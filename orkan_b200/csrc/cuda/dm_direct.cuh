@@ -82,7 +82,7 @@ struct DirectSuper1 {
         }
     }
 };
-// Controlled flip (X, Y, CX, CY, CCX): rows that have all control bits exchange with phases p0 (new target
+// Controlled flip (X, CX, CCX, and any other phases of the kernel layer): rows that have all control bits exchange with phases p0 (new target
 // bit 0) and p1, columns likewise with the conjugate phases; groups without either stay.  UNIT: both
 // phases are 1 and values only move.
 template <bool UNIT>
@@ -110,6 +110,29 @@ struct DirectFlip {
                 z[2 * i] = cmulc(z[2 * i], p0);
                 z[2 * i + 1] = cmulc(z[2 * i + 1], p1);
             }
+        }
+    }
+};
+
+// Y and CY: as DirectFlip with p0 = -i, p1 = i.  The values move and turn by quarters: no product that would make NaN of
+// an infinity's zero part.
+struct DirectFlipY {
+    unsigned long long ctrl;
+    static ORKAN_HD double2 turn(double2 a) { return c2(-a.y, a.x); }           // times i
+    static ORKAN_HD double2 back(double2 a) { return c2(a.y, -a.x); }           // times -i
+    ORKAN_HD bool active(idx_t r0, idx_t c0) const { return (r0 & ctrl) == ctrl || (c0 & ctrl) == ctrl; }
+    ORKAN_HD void apply(const double2 (&x)[4], double2 (&z)[4], idx_t r0, idx_t c0, bool) const {
+        const bool cr = (r0 & ctrl) == ctrl, cc = (c0 & ctrl) == ctrl;
+        double2 y[4];
+#pragma unroll
+        for (unsigned j = 0; j < 2; ++j) {
+            y[j] = cr ? back(x[2 + j]) : x[j];
+            y[2 + j] = cr ? turn(x[j]) : x[2 + j];
+        }
+#pragma unroll
+        for (unsigned i = 0; i < 2; ++i) {
+            z[2 * i] = cc ? turn(y[2 * i + 1]) : y[2 * i];
+            z[2 * i + 1] = cc ? back(y[2 * i]) : y[2 * i + 1];
         }
     }
 };

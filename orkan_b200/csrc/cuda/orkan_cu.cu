@@ -392,6 +392,8 @@ int orkan_cu_dm_monomial(int layout, unsigned log_tile, void* rho, unsigned n, u
         const double2 p0 = op.phase[m - 2], p1 = op.phase[m - 1];
         if (p0.x == 1.0 && p0.y == 0.0 && p1.x == 1.0 && p1.y == 0.0)
             return launch_direct(layout, log_tile, rho, n, qubits[k - 1], DirectFlip<true>{ctrl, p0, p1}, as_stream(stream));
+        if (p0.x == 0.0 && p0.y == -1.0 && p1.x == 0.0 && p1.y == 1.0)
+            return launch_direct(layout, log_tile, rho, n, qubits[k - 1], DirectFlipY{ctrl}, as_stream(stream));
         return launch_direct(layout, log_tile, rho, n, qubits[k - 1], DirectFlip<false>{ctrl, p0, p1}, as_stream(stream));
     }
     DmGeom g;
