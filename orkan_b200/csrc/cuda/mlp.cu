@@ -915,6 +915,15 @@ int rows_backward(orkan_mlp* m, const float* x, const float* t, int rows, float*
     return (int)cudaGetLastError();
 }
 
+// Do the arrays of na floats at a and nb floats at b share memory?  The row kernel writes results of some rows while
+// others are still to be read, so results that lie on its inputs go through the network's own buffers.
+bool overlap(const float* a, size_t na, const float* b, size_t nb) {
+    return a && b && a < b + nb && b < a + na;
+}
+int copy_out(float* dst, const float* src, size_t count, cudaStream_t st) {
+    return (int)cudaMemcpyAsync(dst, src, count * sizeof(float), cudaMemcpyDeviceToDevice, st);
+}
+
 // One training step on the minibatch of the device step counter (captured into a graph).
 void train_step(orkan_mlp* m, const float* X, const float* T, unsigned count, int batch, unsigned spe, uint64_t seed,
                 float lr, cudaStream_t st) {
@@ -1037,18 +1046,24 @@ int orkan_mlp_set_params(orkan_mlp_t* m, const float* host) {
 
 int orkan_mlp_forward(orkan_mlp_t* m, const float* x_dev, unsigned batch, float* y_dev, void* stream) {
     if (!m || !x_dev || !y_dev || batch == 0 || (int)batch > m->maxb) return (int)cudaErrorInvalidValue;
-    if (m->fused) return rows_forward(m, x_dev, (int)batch, y_dev, reinterpret_cast<cudaStream_t>(stream));
-    forward(m, x_dev, (int)batch, y_dev, reinterpret_cast<cudaStream_t>(stream));
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (m->fused) {
+        const bool own = overlap(y_dev, batch, x_dev, (size_t)batch * m->n_in);
+        const int rc = rows_forward(m, x_dev, (int)batch, own ? m->y : y_dev, st);
+        return rc || !own ? rc : copy_out(y_dev, m->y, batch, st);
+    }
+    forward(m, x_dev, (int)batch, y_dev, st);
     return (int)cudaGetLastError();
 }
 
 int orkan_mlp_predict(orkan_mlp_t* m, const float* x_dev, unsigned count, float* y_dev, void* stream) {
     if (!m || !x_dev || !y_dev || count == 0) return (int)cudaErrorInvalidValue;
     // the fused form needs no activations in memory: any count at once, in int-sized pieces
-    const unsigned most = m->fused ? 1u << 24 : (unsigned)m->maxb;
+    const bool whole = m->fused && !overlap(y_dev, count, x_dev, (size_t)count * m->n_in);
+    const unsigned most = whole ? 1u << 24 : (unsigned)m->maxb;
     int rc = 0;
     for (unsigned c0 = 0; c0 < count && !rc; c0 += std::min(most, count - c0))
-        rc = m->fused ? rows_forward(m, x_dev + (size_t)c0 * m->n_in, (int)std::min(most, count - c0), y_dev + c0,
+        rc = whole ? rows_forward(m, x_dev + (size_t)c0 * m->n_in, (int)std::min(most, count - c0), y_dev + c0,
                                      reinterpret_cast<cudaStream_t>(stream))
                       : orkan_mlp_forward(m, x_dev + (size_t)c0 * m->n_in, std::min(most, count - c0), y_dev + c0, stream);
     return rc;
@@ -1058,7 +1073,12 @@ int orkan_mlp_gradients(orkan_mlp_t* m, const float* x_dev, const float* t_dev, 
                         float* grad_dev, float* gx_dev, void* stream) {
     if (!m || !x_dev || !t_dev || !grad_dev || batch == 0 || (int)batch > m->maxb) return (int)cudaErrorInvalidValue;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (m->fused) return rows_backward(m, x_dev, t_dev, (int)batch, loss_dev, grad_dev, gx_dev, st);
+    if (m->fused) {
+        const size_t nx = (size_t)batch * m->n_in;
+        const bool own = overlap(gx_dev, nx, x_dev, nx) || overlap(gx_dev, nx, t_dev, batch);
+        const int rc = rows_backward(m, x_dev, t_dev, (int)batch, loss_dev, grad_dev, own ? m->xb : gx_dev, st);
+        return rc || !own ? rc : copy_out(gx_dev, m->xb, nx, st);
+    }
     forward(m, x_dev, (int)batch, m->y, st);
     k_loss<<<1, 1024, 0, st>>>(m->y, t_dev, (int)batch, m->dy, loss_dev);
     ++g_launches;
