@@ -49,7 +49,8 @@ def test_flips_only_move_values(request, lt, kind, n):
     rho = matrix(n, rng)
     start = R.to_storage(kind, rho, lt)
     st = ork.state(kind, n)
-    cases = [(g, [q], None) for g in "xy" for q in range(n)]
+    some = range(n) if n < 11 else (0, 5, 10)              # below, on and above a tile of 32 groups
+    cases = [(g, [q], None) for g in "xy" for q in some]
     cases += [(g, [c, t], c) for g in ("cx", "cy") for c, t in ((0, n - 1), (n - 1, 0), (n // 2, 0)) if c != t]
     for g, qs, control in cases:
         ork.upload(st, start)

@@ -49,3 +49,35 @@ def test_engine_forms(request, lt, kind, n):
         hook(0, 0)
     assert ork.lib.orkan_cu_engine_status() == 0
     ork.free(st)
+
+
+@pytest.mark.parametrize("kind", ["packed", "tiled"])
+def test_engine_blocks_of_many_items(ork5, kind):
+    """12 qubits are 2080 blocks of 64 x 64 for at most 444 resident ones: each takes several in turn.  Against the
+    direct kernels on the same state."""
+    hook = ork5.lib.orkan_cu_engine_test_wait
+    hook.argtypes, hook.restype = [C.c_ulonglong, C.c_int], None
+    ork5.lib.orkan_cu_engine_status.restype = C.c_uint
+    n = 12
+    st = ork5.plus(kind, n)
+    for q in range(n):
+        ork5.gate(st, "ry", [q], 0.3 + 0.2 * q)
+        ork5.gate(st, "rz", [q], 0.7 - 0.1 * q)
+    sop = R.kraus_to_superop(R.depolarizing_kraus(0.05))
+    ops = [lambda s, q=q, g=g: ork5.gate(s, g, [(q + 7) % n, q] if g[0] == "c" else [q], 0.9 if g == "rx" else None)
+           for g in ("h", "rx", "x", "y", "cx", "cy") for q in (0, 5, 11)]
+    ops += [lambda s, q=q: ork5.channel_1q(s, sop, q) for q in (0, 5, 11)]
+    for op in ops:
+        want, got = ork5.copy(st), ork5.copy(st)
+        op(want)
+        hook(1 << 24, 0)
+        try:
+            op(got)
+            ork5.sync()
+        finally:
+            hook(0, 0)
+        assert np.abs(ork5.storage(got) - ork5.storage(want)).max() <= TOL
+        ork5.free(want)
+        ork5.free(got)
+    assert ork5.lib.orkan_cu_engine_status() == 0
+    ork5.free(st)
