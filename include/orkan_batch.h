@@ -48,7 +48,8 @@ int orkan_qaoa_create(orkan_qaoa_t **out, unsigned count, const unsigned *n_qubi
 
 /* Evaluate every instance: gammas and betas are host arrays [count][p] in instance order;
  * means[i] receives the expectation value of the cost.  Synchronises the stream.  Returns
- * cudaErrorLaunchTimeout when a kernel's bounded wait for staged data ran out. */
+ * cudaErrorLaunchTimeout when a kernel's bounded wait for staged data ran out; the next run starts
+ * afresh. */
 int orkan_qaoa_run(orkan_qaoa_t *b, const double *gammas, const double *betas, double *means, void *stream);
 
 /* Autotune chunk size, block size and buffer depth per qubit count on this batch (timing

@@ -38,7 +38,9 @@ int orkan_mlp_set_params(orkan_mlp_t *m, const float *host);      /* also resets
 int orkan_mlp_forward(orkan_mlp_t *m, const float *x_dev, unsigned batch, float *y_dev, void *stream);
 
 /* The same for any count, in pieces of max_batch where the network's size needs scratch for the
- * activations (256 hidden units and at most 64 inputs need none). */
+ * activations (256 hidden units and at most 64 inputs need none).  The order of the sums, and so the
+ * last bits of f(x), depends on the number of rows of a call: calls of up to 2368 rows add a row's
+ * products in four parts, larger ones in one.  Outputs may lie on the inputs. */
 int orkan_mlp_predict(orkan_mlp_t *m, const float *x_dev, unsigned count, float *y_dev, void *stream);
 
 /* Loss L = mean_b (f(x_b) - t_b)^2 and its gradients: grad_dev (param_count floats, the

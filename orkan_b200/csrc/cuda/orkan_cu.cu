@@ -135,7 +135,7 @@ bool direct_wins(int layout, unsigned n, unsigned q, bool mixes) {
     return layout == 1 || n < 14 || q + (mixes ? 2u : 1u) < n;
 }
 // SWAP: one thread per element while the matrix lies in L2 (11 q: 16.5 against 22.7 us packed, 20.8 against 22.4
-// tiled; 12 q: 64 against 71, 99 against 66).
+// tiled; 12 q: 64 against 71, 99 against 66).  One line for both layouts: packed would gain a tenth at 12 q alone.
 constexpr unsigned kDirectSwap = 11;
 
 // Largest engine block side when at most one gate qubit lies above the sub-tile (a power of
@@ -477,7 +477,8 @@ int orkan_cu_dm_channels(int layout, unsigned log_tile, void* rho, unsigned n, u
     unsigned qs[40], k = 0;
     for (unsigned q = 0; q < n; ++q)
         if (has[q]) qs[k++] = q;
-    // chains of as many of the lowest remaining qubits as fit one staged block
+    // chains of as many of the lowest remaining qubits as fit one staged block; a qubit left over goes to the engine
+    // like them (up to 12 qubits a direct launch would be shorter for it: 14.5 against 20.7 us at 11, equal at 13)
     const unsigned ls_max = ls_max_for(layout, log_tile);
     for (unsigned at = 0; at < k;) {
         DmGeom g;

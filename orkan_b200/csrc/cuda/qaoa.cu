@@ -155,9 +155,10 @@ struct PassShape {
 };
 
 // One pass over the items of a launch.  Block b takes items b, b + grid, ... in turn; group g
-// computes every kGroups-th of them, and the staging warp keeps the free buffers filled: low
+// computes every kGroups-th of them, and the staging warps keep the free buffers filled: low
 // items by one bulk copy of 2^C amplitudes, high items by 16-byte copies of runs.  A group
-// hands its buffer back as soon as its last stage has its amplitudes in registers.
+// hands its buffer back as soon as its last stage has its amplitudes in registers; no such
+// stage reads the phase table that goes back with them (qaoa_pass_setup).
 //
 // Bound: HBM (32 bytes per stored amplitude in a middle pass) and shared memory (2 m - 1
 // stages of 32 bytes) are close at C = 12; the registers of the 16 computing warps leave one
